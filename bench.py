@@ -938,8 +938,8 @@ def main():
     ap.add_argument("--no-accuracy", action="store_true",
                     help="skip the accuracy leg (GPU forms against the oracles)")
     ap.add_argument("--tile", type=int, default=-1,
-                    help="pin the insertion kernel (0-3 register tiles, 4 staged column, 6 pixel-major, "
-                         "5 barrier-free column, -2 scatter); default: library choice")
+                    help="pin the insertion kernel (0-3 register tiles, 4 staged column, 5 or 6 the "
+                         "mode's default kernel, -2 scatter); default: library choice")
     args = ap.parse_args()
     wl = WORKLOADS[args.workload]
     ws, rank, local = dist_setup()
@@ -984,9 +984,10 @@ def main():
     V = (N // 2 + 1) * N * N
     alg_bytes = args.batch * (8 * (N // 2 + 1) * N + 64) + 24 * V
     if st["gather_launches"] > 0:
-        # the library's default: k_column3 for gauss_5, k_pixel for the narrow windows
-        tile = args.tile if args.tile != -1 else (5 if wl["mode"] == "gauss_5" else 6)
-        kname = {6: "k_pixel", 5: "k_column3", 4: "k_column"}.get(tile, "k_gather") + \
+        # the library's default: k_plane, and k_pixel for the narrow windows of large volumes
+        plane = wl["mode"] == "gauss_5" or (wl["mode"] != "nearest_neighbor" and N <= 352)
+        tile = args.tile if args.tile not in (-1, 5, 6) else (5 if plane else 6)
+        kname = {6: "k_pixel", 5: "k_plane", 4: "k_column"}.get(tile, "k_gather") + \
             " (gather schedule)"
         gms = st["gather_ms"] / st["gather_launches"]
     else:

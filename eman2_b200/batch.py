@@ -67,7 +67,7 @@ def insert_particles_multi(recons, images, metas, stream=None):
 
 
 TILE_NAMES = {0: "gather 8x8x8", 1: "gather 16x8x8", 2: "gather 8x8x4", 3: "gather 16x16x4",
-              4: "column (staged)", 5: "column (barrier-free)", 6: "pixel-major", -2: "scatter"}
+              4: "column (staged)", 5: "plane columns", 6: "pixel-major", -2: "scatter"}
 
 
 def autotune(N: int, mode: str, nsym: int, nparticles: int = 256):

@@ -404,6 +404,8 @@ InsertJob make_job(fr_recon *r, const float2 *slices, const float *t3d, const fl
   memset(&j, 0, sizeof j);   // padding too: jobs are compared bytewise for reuse
   j.data = r->vol_data.as<float>();
   j.norm = r->vol_norm.as<float>();
+  j.fdata = j.data;
+  j.fnorm = j.norm;
   j.slices = slices;
   j.t3d = t3d;
   j.pw = pw;
@@ -424,6 +426,7 @@ InsertJob make_job(fr_recon *r, const float2 *slices, const float *t3d, const fl
   j.np = np;
   j.tiles_x = j.tiles_y = j.tiles_z = 0;
   j.nz = r->NZ != r->N ? r->NZ : 0;
+  j.corners = r->p.corners ? 1 : 0;
   return j;
 }
 
@@ -440,6 +443,44 @@ int run_scatter(const InsertJob &j0, bool edge_only, cudaStream_t st) {
     if (j0.wsnr) j.wsnr = j0.wsnr + (size_t)p0 * j0.nwsnr;
     if (j0.wundo) j.wundo = j0.wundo + p0;
     CU(edge_only ? launch_edge(j, st) : launch_scatter(j, st));
+  }
+  return FR_OK;
+}
+
+void PlaneBufs::ensure(int N, long slices, cudaStream_t st) {
+  int half, copies;
+  centre.ensure_zero(plane_centre(N, slices, half, copies), st);
+  if (plane_partial(N, slices))
+    (void)(data.ensure_zero(vol_floats(N) * sizeof(float), st) &&
+           norm.ensure_zero(norm_floats(N) * sizeof(float), st));
+}
+
+int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st) {
+  const long slices = (long)j0.np * j0.nsym;
+  const int N = j0.N;
+  InsertJob j = j0;
+  int half;
+  const size_t cbytes = plane_centre(N, slices, half, j.copies);
+  if (cbytes && !plane_small(j.mode, N, slices) && b.centre.cap >= cbytes) {
+    j.cdata = b.centre.as<float>();
+    j.centre = half;
+  }
+  const bool part = plane_partial(N, slices) && b.data.cap >= vol_floats(N) * sizeof(float) &&
+                    b.norm.cap >= norm_floats(N) * sizeof(float);
+  if (part) {
+    j.data = b.data.as<float>();
+    j.norm = b.norm.as<float>();
+  }
+  const long turns = part || j.cdata ? (slices + kPlaneTurn - 1) / kPlaneTurn : 1;
+  const int per = (int)((j0.np + turns - 1) / turns);
+  for (int p0 = 0; p0 < j0.np; p0 += per) {
+    j.np = std::min(per, j0.np - p0);
+    j.slices = j0.slices + (size_t)p0 * N * (N / 2 + 1);
+    j.t3d = j0.t3d + (size_t)p0 * j0.nsym * 9;
+    j.pw = j0.pw + p0;
+    CU(launch_plane(j, st));
+    if (j.cdata) CU(launch_merge_centre(nullptr, 1, &j, j.mode, j.centre, st));
+    if (part) CU(launch_merge(j0.data, j0.norm, j.data, j.norm, N, j0.corners, st));
   }
   return FR_OK;
 }
@@ -473,9 +514,23 @@ int insert_device(fr_recon *r, const float2 *d_slices, const float *d_t3d, const
     for (auto &e : ev) CU(cudaEventCreate(&e));
   g_ins_launches++;
   g_slices += (long long)np * r->nsym;
-  if (sched == FR_SCHED_SCATTER || d_ssnr) {
+  // the tile of a gather call; the plane-column kernel also takes the calls
+  // the scatter schedule names, unless they need its per-pixel weights or its
+  // z size
+  int tile = r->tile >= 0 ? r->tile : (tuned >= 0 ? tuned : default_tile(r->mode, r->N, r->nsym, np));
+  tile = effective_tile(tile, r->mode, r->N);
+  const bool gather = sched != FR_SCHED_SCATTER && !d_ssnr;
+  const bool plane = plane_mode(r->mode) && r->NZ == r->N && !d_ssnr &&
+                     (!gather || tile == kPlaneTile);
+  if (plane || !gather) {
     if (prof) CU(cudaEventRecord(ev[0], st));
-    TRY(run_scatter(j, false, st));
+    if (plane) {
+      r->plane.ensure(r->N, (long)np * r->nsym, st);
+      TRY(run_plane(j, r->plane, st));
+    } else {
+      TRY(run_scatter(j, false, st));
+    }
+    if (gather) g_gather_launches++;
     if (prof) {
       CU(cudaEventRecord(ev[2], st));
       CU(cudaEventSynchronize(ev[2]));
@@ -483,12 +538,11 @@ int insert_device(fr_recon *r, const float2 *d_slices, const float *d_t3d, const
       cudaEventElapsedTime(&ms, ev[0], ev[2]);
       std::lock_guard<std::mutex> lk(g_stat_mu);
       g_insert_ms += ms;
+      if (gather) g_gather_ms += ms;
       for (auto &e : ev) cudaEventDestroy(e);
     }
     return FR_OK;
   }
-  int tile = r->tile >= 0 ? r->tile : (tuned >= 0 ? tuned : default_tile(r->mode, r->N, r->nsym, np));
-  tile = effective_tile(tile, r->mode);
   if (r->tiles_tile != tile) {
     if (is_column_tile(tile))
       column_tiles(r->N, r->mode, r->p.corners, r->tiles, r->tx, r->ty, r->tz, &r->tile_dist);
@@ -553,9 +607,6 @@ int insert_device(fr_recon *r, const float2 *d_slices, const float *d_t3d, const
   if (tile == kPixelTile)
     CU(launch_pixel(d_job, r->s_work.as<int4>(), nwork, kColumnBlock,
                     r->s_counter.as<int>(), r->N, st));
-  else if (tile == kColumn3Tile)
-    CU(launch_column3(d_job, r->s_work.as<int4>(), nwork, kColumnBlock,
-                      r->s_counter.as<int>(), r->N, st));
   else if (tile == kColumnTile)
     CU(launch_column(d_job, r->s_work.as<int4>(), nwork, kColumnBlock,
                      r->s_counter.as<int>(), r->mode, st));
@@ -820,6 +871,7 @@ int fr_destroy(fr_recon *r) {
                       &r->s_txy, &r->s_out, &r->s_ssnr, &r->s_jobs, &r->s_work,
                       &r->s_counter};
     for (DevBuf *b : bufs) b->release();
+    r->plane.release();
     for (int k = 0; k < 2; k++) {
       r->s_stage[k].release();
       if (r->staged[k]) cudaEventDestroy(r->staged[k]);

@@ -38,10 +38,8 @@ int tuned_tile(int N, int mode, int nsym) {
 }
 
 int default_tile(int mode, int N, int nsym, int np) {
-  (void)nsym; (void)np; (void)N; (void)mode;
-  // unless the autotuner measured otherwise: the pixel-major kernel for the
-  // narrow windows, the barrier-free column kernel for gauss_5
-  return mode == FR_MODE_GAUSS5 ? kColumn3Tile : kPixelTile;
+  (void)nsym; (void)np;
+  return effective_tile(kPlaneTile, mode, N);   // unless the autotuner measured otherwise
 }
 
 }  // namespace fr
@@ -71,6 +69,7 @@ struct ProBufs {
 struct BatchScratch {
   DevBuf d_jobs, d_work, d_counter, d_meta;
   std::vector<ProBufs> gbufs;
+  std::vector<PlaneBufs> plane;   // per schedule group (groups may run concurrently)
   PinnedRing ring;
   cudaEvent_t done = nullptr;     // after the last launch that read this scratch
   cudaStream_t last = nullptr;
@@ -79,6 +78,8 @@ struct BatchScratch {
     for (DevBuf *b : {&d_jobs, &d_work, &d_counter, &d_meta}) b->release();
     for (ProBufs &g : gbufs) g.release();
     gbufs.clear();
+    for (PlaneBufs &v : plane) v.release();
+    plane.clear();
     ring.release();
   }
   ~BatchScratch() { release(); }
@@ -165,6 +166,17 @@ struct RoundGroup {
   // gather launch: offset in the work buffer, count, largest pixel (rim) count
   size_t units_off = 0, nunits = 0;
   int max_px = 0;
+  // a plane-column group: the jobs that go through a partial volume, one
+  // after another (those of many slices, then any the shared launch's unit
+  // count has no room for), and the others' segments (offset and count at
+  // units_off, nunits) with the launch's unit count
+  std::vector<int> turns;
+  int units = 0;
+  // the segments' centre copies: offset of each (job, bytes from the start of
+  // the group's buffer), their total and the largest half-width
+  std::vector<std::pair<int, size_t>> centres;
+  size_t centre_bytes = 0;
+  int centre_half = 0;
 };
 struct RoundPlan {
   std::vector<InsertJob> hj;
@@ -175,13 +187,19 @@ struct RoundPlan {
 
 static bool is_column(int tile) { return is_column_tile(tile); }
 
+// The plane-column jobs of one mode form a group of their own.
+constexpr int kPlaneGroup = 1000;
+static bool is_plane_group(int tile) { return tile >= kPlaneGroup; }
+
 // Each job's schedule: the caller's pin, else the autotuner's measurement for
-// its (N, mode, nsym), else the barrier-free column kernel.  Jobs that share
+// its (N, mode, nsym), else the default kernel of its mode.  Jobs that share
 // a schedule share one persistent launch per round.
 static int job_tile(const fr_recon *r, int tile_pref) {
-  if (tile_pref != -1) return effective_tile(tile_pref, r->mode);
-  const int t = tuned_tile(r->N, r->mode, r->nsym);
-  return effective_tile(t != -1 ? t : default_tile(r->mode, r->N, r->nsym, 0), r->mode);
+  int t = tile_pref != -1 ? tile_pref : tuned_tile(r->N, r->mode, r->nsym);
+  if (t == -1) t = default_tile(r->mode, r->N, r->nsym, 0);
+  t = effective_tile(t, r->mode, r->N);
+  if (t == kPlaneTile || (t == kTunedScatter && plane_mode(r->mode))) return kPlaneGroup + r->mode;
+  return t;
 }
 
 // Adds job r's InsertJob (its chunk's np slices, composed rotations and
@@ -190,7 +208,7 @@ static void plan_add(RoundPlan &P, fr_recon *r, int owner, int np, int tile_pref
                      const float2 *slices, const float *t3d, const float *pw) {
   InsertJob J = make_job(r, slices, t3d, pw, np);
   const int tile = job_tile(r, tile_pref);
-  if (tile != kTunedScatter && r->tiles_tile != tile) {
+  if (tile != kTunedScatter && !is_plane_group(tile) && r->tiles_tile != tile) {
     if (is_column(tile))
       column_tiles(r->N, r->mode, r->p.corners, r->tiles, r->tx, r->ty, r->tz, &r->tile_dist);
     else gather_tiles(r->N, r->mode, tile, r->p.corners, r->tiles, r->tx, r->ty, r->tz);
@@ -226,6 +244,37 @@ static void plan_units(RoundPlan &P, RoundGroup &g, bool edge) {
   if (!u.empty()) memcpy(&P.work[g.units_off], u.data(), sizeof(int2) * u.size());
 }
 
+// A plane-column group's jobs: those with enough slices for a partial volume
+// one by one, the others as segments of one launch.
+static void plan_plane(RoundPlan &P, RoundGroup &g) {
+  std::vector<PlaneSeg> segs;
+  g.max_mode = g.tile - kPlaneGroup;
+  for (size_t k = 0; k < P.hj.size(); k++) {
+    if (P.jt[k] != g.tile) continue;
+    const InsertJob &J = P.hj[k];
+    PlaneSeg q;
+    int next = -1;
+    if (!plane_partial(J.N, (long)J.np * J.nsym)) next = plane_seg(J, (int)k, g.units, q);
+    if (next < 0) {
+      g.turns.push_back((int)k);
+      continue;
+    }
+    segs.push_back(q);
+    int half, copies;
+    if (const size_t bytes = plane_centre(J.N, (long)J.np * J.nsym, half, copies)) {
+      g.centres.push_back({(int)k, g.centre_bytes});
+      g.centre_bytes += (bytes + 255) & ~(size_t)255;
+      g.centre_half = std::max(g.centre_half, half);
+    }
+    g.units = next;
+    g.maxN = std::max(g.maxN, J.N);
+  }
+  g.units_off = (P.work.size() + 15) & ~(size_t)15;
+  g.nunits = segs.size();
+  P.work.resize(g.units_off + sizeof(PlaneSeg) * segs.size());
+  if (!segs.empty()) memcpy(&P.work[g.units_off], segs.data(), sizeof(PlaneSeg) * segs.size());
+}
+
 // Builds each schedule group's work list.  Column items run slice-bucket-major
 // (slice_bucket per job, so the CTAs in flight share a bucket's slices in L2)
 // and within a bucket by estimated cost, heaviest first: the slices meeting a
@@ -238,6 +287,11 @@ static void plan_groups(const std::vector<fr_recon *> &jobs, RoundPlan &P) {
   for (const int tile : tiles_used) {
     RoundGroup g;
     g.tile = tile;
+    if (is_plane_group(tile)) {
+      plan_plane(P, g);
+      P.groups.push_back(g);
+      continue;
+    }
     if (tile == kTunedScatter) {
       plan_units(P, g, false);
       P.groups.push_back(g);
@@ -291,11 +345,26 @@ static void plan_groups(const std::vector<fr_recon *> &jobs, RoundPlan &P) {
 }
 
 // Job table and work lists to the device (host sources are pageable
-// vectors: the copies have taken them when cudaMemcpyAsync returns).
-static int plan_upload(const RoundPlan &P, BatchScratch &bs, cudaStream_t st) {
+// vectors: the copies have taken them when cudaMemcpyAsync returns), and the
+// plane groups' workspaces.  The centre copies of a group's shared launch sit
+// one after another; a job that takes turns by itself has all of its own
+// before or after, so it reuses them from the start.
+static int plan_upload(RoundPlan &P, BatchScratch &bs, cudaStream_t st) {
   TRY(bs.d_jobs.ensure(sizeof(InsertJob) * std::max<size_t>(1, P.hj.size())));
   TRY(bs.d_counter.ensure(sizeof(int) * std::max<size_t>(1, P.groups.size())));
   TRY(bs.d_work.ensure(std::max<size_t>(16, P.work.size())));
+  if (bs.plane.size() < P.groups.size()) bs.plane.resize(P.groups.size());
+  for (size_t gi = 0; gi < P.groups.size(); gi++) {
+    RoundGroup &g = P.groups[gi];
+    PlaneBufs &b = bs.plane[gi];
+    for (int k : g.turns) b.ensure(P.hj[k].N, (long)P.hj[k].np * P.hj[k].nsym, st);
+    if (!b.centre.ensure_zero(g.centre_bytes, st)) g.centres.clear();
+    for (const auto &c : g.centres) {
+      InsertJob &J = P.hj[c.first];
+      plane_centre(J.N, (long)J.np * J.nsym, J.centre, J.copies);
+      J.cdata = reinterpret_cast<float *>(b.centre.as<unsigned char>() + c.second);
+    }
+  }
   TRY(bs.ring.upload(bs.d_jobs.p, P.hj.data(), sizeof(InsertJob) * P.hj.size(), st));
   if (!P.work.empty()) TRY(bs.ring.upload(bs.d_work.p, P.work.data(), P.work.size(), st));
   return FR_OK;
@@ -314,11 +383,17 @@ static int plan_launch_group(const RoundPlan &P, BatchScratch &bs, size_t gi, cu
     CU(launch_scatter_multi(d_jobs, units, (int)g.nunits, g.max_px, false, st));
     return FR_OK;
   }
+  if (is_plane_group(g.tile)) {
+    for (int k : g.turns) TRY(run_plane(P.hj[k], bs.plane[gi], st));
+    CU(launch_plane_multi(d_jobs, (const PlaneSeg *)units, (int)g.nunits, g.units, g.max_mode,
+                          g.maxN, st));
+    if (!g.centres.empty())
+      CU(launch_merge_centre(d_jobs, (int)P.hj.size(), nullptr, g.max_mode, g.centre_half, st));
+    return FR_OK;
+  }
   const void *w = (const unsigned char *)bs.d_work.p + g.off;
   if (g.tile == kPixelTile)
     CU(launch_pixel(d_jobs, (const int4 *)w, (int)g.nwork, kColumnBlock, counter, g.maxN, st));
-  else if (g.tile == kColumn3Tile)
-    CU(launch_column3(d_jobs, (const int4 *)w, (int)g.nwork, kColumnBlock, counter, g.maxN, st));
   else if (g.tile == kColumnTile)
     CU(launch_column(d_jobs, (const int4 *)w, (int)g.nwork, kColumnBlock, counter, g.max_mode, st));
   else
@@ -905,7 +980,7 @@ int fr_set_tile(int N, int mode, int nsym, int tile) {
 // schedule, on random slices of size N through random orientations; records
 // the fastest for (N, mode, nsym).  tile_out: chosen tile (-2 = scatter);
 // ms_out[kPixelTile+2]: per-candidate milliseconds (register tiles 0-3,
-// staged column 4, barrier-free column 5, pixel-major 6 (gauss_5: -1), then
+// staged column 4, the mode's default kernel 5 and 6 (gauss_5: 6 is -1), then
 // scatter).
 int fr_autotune(int N, int mode, int nsym, int nparticles, int *tile_out, float *ms_out) {
   if (nparticles <= 0) return fail(FR_EINVAL_PARAM, "nparticles must be positive");
@@ -957,7 +1032,7 @@ int fr_autotune(int N, int mode, int nsym, int nparticles, int *tile_out, float 
   int measured = 0;
   for (int cand = 0; cand <= kPixelTile + 1 && rc == FR_OK; cand++) {
     const bool scatter = cand == kPixelTile + 1;
-    if (!scatter && effective_tile(cand, mode) != cand) {   // no pixel-major gauss_5
+    if (cand == kPixelTile && mode == FR_MODE_GAUSS5) {   // 5 has run it
       if (ms_out) ms_out[cand] = -1.0f;
       continue;
     }

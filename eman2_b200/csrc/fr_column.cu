@@ -1,4 +1,5 @@
-// fr_column.cu -- the column-owner insertion kernel (gather schedule, v2).
+// fr_column.cu -- the insertion kernels over 16^3 voxel tiles: the staged
+// column-owner kernel (below) and the pixel-major kernel (further down).
 //
 // Work item = (job, 16^3 voxel tile, block of slices).  For each slice of the
 // block whose plane passes the tile, the slice's pixel patch is staged in
@@ -362,403 +363,7 @@ __device__ void tile_item(const InsertJob &J, int tile, int s0, int s1, const Sm
   __syncthreads();
 }
 
-// ------------------------------------------------------------------ v3
-// Barrier-free variant: no patch staging.  Hits are grouped by the column
-// axis A; within a group every thread walks all slices for its own column,
-// computing each candidate pixel's coordinates itself (the same exact
-// operations), so threads never wait for one another until A changes.
-// Three CTAs of 256 threads per SM (24 warps; the kernel is bound by
-// latency, so warps count most): shared memory is the 64 KB accumulator
-// tile plus compact tables (16-bit slice offsets and row limits; the
-// fast_exp table serves gauss_2 too, with the same exact index), ~74 KB.
-struct Smem3 {
-  float4 *acc;      // [NV]
-  float4 *steps;    // (not used by this kernel)
-  float *exp;       // [1000] fast_exp table
-  float *rtab;      // [N+2]
-  short *xmax;      // [N]
-  unsigned short *hits;  // [block] slice - s0, grouped by axis
-  unsigned short *tmp;   // [block] (slice - s0) | group << 14
-  int *wcount;      // [3 * NT/32]
-  int *gcount;      // [3]
-  int *state;       // [0] steps mode loaded, [1] job geometry loaded (N)
-};
-constexpr int STEP2CAP = 800;   // gauss_2 step table entries (K = 256 over r <= 3.01: 772)
-
-// Tile-local coordinates (x, y, z) of cell i in layout L: L = A holds the
-// tile A-major, (a, b, c) at a*T*T + c*T + b with b < c the other two axes;
-// layout 2 is the volume's own [z][y][x] order.
-__device__ __forceinline__ void tile_cell(int L, int i, int *l) {
-  const int a = i >> 8, c = (i >> 4) & 15, b = i & 15;
-  if (L == 0) { l[0] = a; l[1] = b; l[2] = c; }
-  else if (L == 1) { l[0] = b; l[1] = a; l[2] = c; }
-  else { l[0] = b; l[1] = c; l[2] = a; }
-}
-__device__ __forceinline__ int tile_index(int L, const int *l) {
-  if (L == 0) return (l[0] << 8) | (l[2] << 4) | l[1];
-  if (L == 1) return (l[1] << 8) | (l[2] << 4) | l[0];
-  return (l[2] << 8) | (l[1] << 4) | l[0];
-}
-// Moves the tile's accumulators from layout `from` to layout `to` (all
-// threads; barriers inside).  Layouts 0 -> 1 swap the x and y digits of the
-// cell index, 1 -> 2 the y and z digits: each an involution, done as pair
-// swaps with no scratch; 0 -> 2 is both.
-__device__ __forceinline__ void swap_digits(float4 *acc, int hi_shift, int lo_shift) {
-  // cells (.., u at hi_shift, .., v at lo_shift, ..) <-> (.., v, .., u, ..), u < v
-  for (int i = threadIdx.x; i < NV; i += blockDim.x) {
-    const int u = (i >> hi_shift) & 15, v = (i >> lo_shift) & 15;
-    if (u < v) {
-      const int j = i + ((v - u) << hi_shift) - ((v - u) << lo_shift);
-      const float4 a = acc[i];
-      acc[i] = acc[j];
-      acc[j] = a;
-    }
-  }
-}
-__device__ __noinline__ void relayout(float4 *acc, int from, int to) {
-  __syncthreads();
-  if (from == 0) {          // L0 = x:8, z:4, y:0  ->  L1 = y:8, z:4, x:0
-    swap_digits(acc, 8, 0);
-    __syncthreads();
-    from = 1;
-  }
-  if (from == 1 && to == 2) {   // L1 = y:8, z:4, x:0  ->  L2 = z:8, y:4, x:0
-    swap_digits(acc, 8, 4);
-    __syncthreads();
-  }
-}
-
-template <int MODE, int A>
-__device__ __forceinline__ void column_work(const Smem3 &S, const float *M, int sg, const int *base,
-                                            const int *ext, int N, const float2 *__restrict__ sl,
-                                            float w, float h, const ExpSteps &steps) {
-  constexpr int B = (A == 0) ? 1 : 0;
-  constexpr int C = (A == 2) ? 1 : 2;
-  constexpr float RLO = Win<MODE>::lo, RHI = Win<MODE>::hi;
-  constexpr int K = Win<MODE>::K;
-  const int n2 = N >> 1;
-  const float Nf = (float)N;
-  const float *m0 = M, *m1 = M + 3, *nrm = M + 6;
-  // A warp's 32 columns are an 8 x 4 patch of the tile's (b, c) face: the
-  // band of columns a slice's plane reaches in a tile cuts compact patches
-  // less often than 16 x 2 strips, so fewer lanes idle (a model of every
-  // tile a slice meets: 65 % of a warp's tap slots used against 57 %).
-  const int wl = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const int lb = (wl & 7) + ((wp & 1) << 3), lc = (wl >> 3) + ((wp >> 1) << 2);
-  const int vb = base[B] + lb, vc = base[C] + lc;
-  if (vb > ext[B] || vc > ext[C]) return;
-  const int tb = sg * vb, tc = sg * vc;
-  const int ta_lo = sg > 0 ? base[A] : -ext[A];
-  const int ta_hi = sg > 0 ? ext[A] : -base[A];
-  float lo[3], hi[3];
-  lo[A] = ta_lo - RLO - kDel; hi[A] = ta_hi + RHI + kDel;
-  lo[B] = tb - RLO - kDel;    hi[B] = tb + RHI + kDel;
-  lo[C] = tc - RLO - kDel;    hi[C] = tc + RHI + kDel;
-  // quick reject: heights of the plane over the column's (b, c) window
-  {
-    const float ia = 1.0f / nrm[A];
-    float pmin = 1e30f, pmax = -1e30f;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float pb = (i & 1) ? hi[B] : lo[B], pc = (i & 2) ? hi[C] : lo[C];
-      const float pa = -(nrm[B] * pb + nrm[C] * pc) * ia;
-      pmin = fminf(pmin, pa);
-      pmax = fmaxf(pmax, pa);
-    }
-    if (pmax < lo[A] - 0.05f || pmin > hi[A] + 0.05f) return;
-  }
-  const float det = m0[B] * m1[C] - m0[C] * m1[B];
-  const float idet = 1.0f / det;
-  float ymin = 1e30f, ymax = -1e30f;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const float pb = (i & 1) ? hi[B] : lo[B], pc = (i & 2) ? hi[C] : lo[C];
-    const float y = (m0[B] * pc - m0[C] * pb) * idet;
-    ymin = fminf(ymin, y);
-    ymax = fmaxf(ymax, y);
-  }
-  const int r0 = max(-n2, (int)ceilf(ymin)), r1 = min(n2 - 1, (int)floorf(ymax));
-  float inv0[3];
-#pragma unroll
-  for (int a = 0; a < 3; a++) inv0[a] = fabsf(m0[a]) > 1e-4f ? 1.0f / m0[a] : 0.0f;
-  // The tile is held A-major while group A runs: cell (a, b, c) of the tile
-  // at a*T*T + c*T + b, so a thread's column is c*T + b + a*T*T; each quarter
-  // warp holds 8 consecutive b of one c, so a warp's float4 accesses take the
-  // minimum 4 shared wavefronts whatever taps its lanes add.
-  const int col_addr = lc * T + lb;
-  const bool xzero_col = (A != 0) && (vb == 0);
-  for (int y = r0; y <= r1; y++) {
-    const int xm = S.xmax[y + n2];
-    float xlo = 0.f, xhi = (float)xm;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const float c = m1[a] * (float)y;
-      const float L = lo[a] - c, U = hi[a] - c;
-      if (inv0[a] > 0.f) { xlo = fmaxf(xlo, L * inv0[a]); xhi = fminf(xhi, U * inv0[a]); }
-      else if (inv0[a] < 0.f) { xlo = fmaxf(xlo, U * inv0[a]); xhi = fminf(xhi, L * inv0[a]); }
-      else if (L > 0.05f || U < -0.05f) xhi = -1e30f;
-    }
-    const int c0 = max(0, (int)ceilf(xlo)), c1 = min(xm, (int)floorf(xhi));
-    if (c0 > c1) continue;
-    const float ry = S.rtab[y + n2];
-    // the row's slice values; pixel (0, y < 0) reads (0, -y) conjugated
-    const int w2s = (N >> 1) + 1;
-    const float2 *rowp = sl + (size_t)(y < 0 ? N + y : y) * w2s;
-    const float2 *mirp = sl + (size_t)(y < 0 ? -y : 0) * w2s;
-    for (int x = c0; x <= c1; x++) {
-      float xx, yy, zz;
-      pixel_coords(S.rtab[x + n2], ry, M, Nf, xx, yy, zz);
-      const float pa = A == 0 ? xx : (A == 1 ? yy : zz);
-      const float pb = B == 0 ? xx : yy;
-      const float pc = C == 1 ? yy : zz;
-      if (!(in_win<MODE>(tb, pb) && in_win<MODE>(tc, pc))) continue;
-      const int a0 = win_start<MODE>(pa);
-      const int k0 = max(a0, ta_lo), k1 = min(a0 + K - 1, ta_hi);
-      if (k0 > k1) continue;
-      const bool herm = (x == 0) && (y < 0);
-      float2 v = __ldg(herm ? mirp : rowp + x);
-      if (herm) v.y = -v.y;
-      float f0 = 0.f, f1 = 0.f;
-      if (MODE == MODE_GAUSS2 || MODE == MODE_GAUSS5) {
-        if (A == 0) {
-          const float dy = __fsub_rn((float)tb, yy), dz = __fsub_rn((float)tc, zz);
-          f0 = __fmul_rn(dy, dy); f1 = __fmul_rn(dz, dz);
-        } else if (A == 1) {
-          const float dx = __fsub_rn((float)tb, xx), dz = __fsub_rn((float)tc, zz);
-          f0 = __fmul_rn(dx, dx); f1 = __fmul_rn(dz, dz);
-        } else {
-          const float dx = __fsub_rn((float)tb, xx), dy = __fsub_rn((float)tc, yy);
-          f0 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-        }
-      }
-      // the window's taps along A inside the tile (the rest belong to the
-      // neighbouring tile's work item): a predicated straight line for the
-      // 2-tap windows, a loop for gauss_5's 6 (its unrolled form is slower)
-      auto tap = [&](int k, float kf) {
-        float vre, vim, vw;
-        if (MODE == MODE_GAUSS2 || MODE == MODE_GAUSS5) {
-          const float d = __fsub_rn(kf, pa);
-          const float d2 = __fmul_rn(d, d);
-          float r;
-          if (A == 0) r = __fadd_rn(__fadd_rn(d2, f0), f1);
-          else if (A == 1) r = __fadd_rn(__fadd_rn(f0, d2), f1);
-          else r = __fadd_rn(f0, d2);
-          if (MODE == MODE_GAUSS2) {
-            // r >= 0 and h > 0, so f <= 0: fast_exp's f > 0 branch never runs
-            const float f = __fmul_rn(-r, h);
-            float g = S.exp[min(__double2int_rz(__fma_rn((double)(-f), 50.0, 0.5)), 999)];
-            if (f < -19.98f) g = expf(f);
-            const float gg = __fmul_rn(g, w);
-            vre = __fmul_rn(v.x, gg);
-            vim = __fmul_rn(v.y, gg);
-            vw = gg;
-          } else {
-            // Util::fast_exp(f): the table index (int)(-f*50.0+0.5) is formed
-            // in double as the reference forms it; -f*50 + 0.5 is exact in
-            // double (a float times 50 plus 0.5 needs at most 31 bits), so
-            // one DFMA and a truncating conversion give the reference's index.
-            // The entry is read for every tap (index clamped to the table) and
-            // replaced by exp(f) past it, so the common path has no branch;
-            // f <= 0 always (r >= 0, h > 0).
-            const float f = __fmul_rn(-r, h);
-            float gg = S.exp[min(__double2int_rz(__fma_rn((double)(-f), 50.0, 0.5)), 999)];
-            if (f < -19.98f) gg = expf(f);
-            vre = __fmul_rn(__fmul_rn(v.x, gg), w);
-            vim = __fmul_rn(__fmul_rn(v.y, gg), w);
-            vw = __fmul_rn(gg, w);
-          }
-        } else {
-          int t[3];
-          t[A] = k; t[B] = tb; t[C] = tc;
-          tap_value<MODE>(t[0], t[1], t[2], xx, yy, zz, v.x, v.y, w, h, nullptr, vre, vim, vw);
-        }
-        const int la = sg * k - base[A];
-        float4 *cell = &S.acc[col_addr + la * (T * T)];
-        float4 u = *cell;
-        const bool origin = (k == 0 && tb == 0 && tc == 0);
-        if (sg > 0) {
-          u.x += vre;
-          if (origin) u.w = 1.0f;
-          else u.y += vim;
-          u.z += vw;
-        } else {
-          if (origin) return;
-          u.x += vre;
-          u.y -= vim;
-          const bool xzero = (A == 0) ? (k == 0) : xzero_col;
-          if (!xzero) u.z += vw;
-        }
-        *cell = u;
-      };
-      if (K <= 2) {
-#pragma unroll
-        for (int j = 0; j < K; j++) {
-          const int k = a0 + j;
-          if (k >= k0 && k <= k1) tap(k, (float)k);
-        }
-      } else {
-        float kf = (float)k0;   // exact: |k| < 2^24
-        for (int k = k0; k <= k1; k++, kf += 1.0f) tap(k, kf);
-      }
-    }
-  }
-}
-
-template <int MODE, int A>
-__device__ __forceinline__ void group_work(const InsertJob &J, const Smem3 &S, int g0, int g1,
-                                           const int *base, const int *ext, float h,
-                                           const ExpSteps &steps, int s0) {
-  const int N = J.N, w2 = (N >> 1) + 1;
-  for (int hI = g0; hI < g1; hI++) {
-    const int s = s0 + S.hits[hI];
-    const int p = s / J.nsym;
-    float M[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) M[i] = __ldg(&J.t3d[9 * s + i]);
-    const float w = __ldg(&J.pw[p]);
-    const float2 *sl = J.slices + (size_t)p * N * w2;
-    column_work<MODE, A>(S, M, 1, base, ext, N, sl, w, h, steps);
-    column_work<MODE, A>(S, M, -1, base, ext, N, sl, w, h, steps);
-  }
-}
-
-template <int MODE>
-__device__ void tile_item3(const InsertJob &J, int tile, int s0, int s1, const Smem3 &S, float h,
-                           const ExpSteps &steps, int *err) {
-  constexpr float RLO = Win<MODE>::lo, RHI = Win<MODE>::hi;
-  const int N = J.N, n2 = N >> 1;
-  const int tix = tile % J.tiles_x, tiy = (tile / J.tiles_x) % J.tiles_y,
-            tiz = tile / (J.tiles_x * J.tiles_y);
-  const int base[3] = {tix * T, -n2 + 1 + tiy * T, -n2 + 1 + tiz * T};
-  const int ext[3] = {min(base[0] + T - 1, n2 - 1), min(base[1] + T - 1, n2 - 1),
-                      min(base[2] + T - 1, n2 - 1)};
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int NW = NT / 32;
-  // ---- cull, and count the hits of each axis group
-  int nhit = 0;
-  for (int r = s0; r < s1; r += NT) {
-    const int s = r + threadIdx.x;
-    int grp = -1;
-    if (s < s1 && __ldg(&J.pw[s / J.nsym]) != 0.0f) {
-      const float n[3] = {__ldg(&J.t3d[9 * s + 6]), __ldg(&J.t3d[9 * s + 7]), __ldg(&J.t3d[9 * s + 8])};
-      // A pixel's direct taps reach the tile from [base - RLO, ext + RHI];
-      // its conjugate taps (mirrored) from [base - RHI, ext + RLO].  The
-      // plane passes through the origin, so one test against the union box
-      // covers both passes (gauss_5's window is asymmetric: 2.5 / 3.5).
-      constexpr float RC = (RLO > RHI ? RLO : RHI) + kDel;
-      const float lo[3] = {base[0] - RC, base[1] - RC, base[2] - RC};
-      const float hi[3] = {ext[0] + RC, ext[1] + RC, ext[2] + RC};
-      float mn, mx;
-      box_dot(n, lo, hi, mn, mx);
-      if (mn <= kPlaneTol && mx >= -kPlaneTol) {
-        const float a0 = fabsf(n[0]), a1 = fabsf(n[1]), a2 = fabsf(n[2]);
-        grp = (a0 >= a1 && a0 >= a2) ? 0 : (a1 >= a2 ? 1 : 2);
-      }
-    }
-    const unsigned b = __ballot_sync(0xffffffffu, grp >= 0);
-    if (lane == 0) S.wcount[warp] = __popc(b);
-    __syncthreads();
-    int off = 0, tot = 0;
-#pragma unroll
-    for (int i = 0; i < NW; i++) {
-      const int c = S.wcount[i];
-      off += (i < warp) ? c : 0;
-      tot += c;
-    }
-    if (grp >= 0) {
-      const int at = nhit + off + __popc(b & ((1u << lane) - 1u));
-      S.tmp[at] = (unsigned short)((s - s0) | (grp << 14));
-    }
-    nhit += tot;
-    __syncthreads();
-  }
-  if (nhit == 0) return;
-  // ---- stable partition of the hits by axis group
-  if (threadIdx.x < 3) S.gcount[threadIdx.x] = 0;
-  __syncthreads();
-  int gstart[4];
-  {
-    int base_g = 0;
-    for (int g = 0; g < 3; g++) {
-      gstart[g] = base_g;
-      for (int r = 0; r < nhit; r += NT) {
-        const int i = r + threadIdx.x;
-        const bool in = i < nhit && (S.tmp[i] >> 14) == g;
-        const unsigned b = __ballot_sync(0xffffffffu, in);
-        if (lane == 0) S.wcount[warp] = __popc(b);
-        __syncthreads();
-        int off = 0, tot = 0;
-#pragma unroll
-        for (int q = 0; q < NW; q++) {
-          const int c = S.wcount[q];
-          off += (q < warp) ? c : 0;
-          tot += c;
-        }
-        if (in) S.hits[base_g + off + __popc(b & ((1u << lane) - 1u))] = S.tmp[i] & 0x3FFF;
-        base_g += tot;
-        __syncthreads();
-      }
-    }
-    gstart[3] = base_g;
-  }
-  // ---- per-job tables and this mode's exp table
-  if (*(S.state + 1) != J.N) {
-    for (int i = threadIdx.x; i < N + 2; i += NT) S.rtab[i] = __ldg(&J.rtab[i]);
-    for (int i = threadIdx.x; i < N; i += NT) S.xmax[i] = (short)__ldg(&J.xmax[i]);
-  }
-  for (int i = threadIdx.x; i < NV; i += NT) S.acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (MODE == MODE_GAUSS2) *S.state = MODE;
-    *(S.state + 1) = J.N;
-  }
-  // ---- the three axis groups; ownership of a voxel changes only between
-  // them, and so does the tile's layout (A-major for group A)
-  int layout = -1;   // -1: nothing added yet, any layout holds the zeros
-  if (gstart[1] > gstart[0]) {
-    group_work<MODE, 0>(J, S, gstart[0], gstart[1], base, ext, h, steps, s0);
-    layout = 0;
-  }
-  __syncthreads();
-  if (gstart[2] > gstart[1]) {
-    if (layout == 0) relayout(S.acc, 0, 1);
-    group_work<MODE, 1>(J, S, gstart[1], gstart[2], base, ext, h, steps, s0);
-    layout = 1;
-  }
-  __syncthreads();
-  if (gstart[3] > gstart[2]) {
-    if (layout == 0 || layout == 1) relayout(S.acc, layout, 2);
-    group_work<MODE, 2>(J, S, gstart[2], gstart[3], base, ext, h, steps, s0);
-    layout = 2;
-  }
-  __syncthreads();
-  // ---- flush
-  const size_t nxf = (size_t)N + 2;
-  const int w2 = n2 + 1;
-  for (int i = threadIdx.x; i < NV; i += NT) {
-    const float4 v = S.acc[i];
-    if (v.x == 0.f && v.y == 0.f && v.z == 0.f && v.w == 0.f) continue;
-    int l3[3];
-    tile_cell(layout, i, l3);
-    const int vx = base[0] + l3[0], vy = base[1] + l3[1], vz = base[2] + l3[2];
-    if (vx > ext[0] || vy > ext[1] || vz > ext[2]) continue;
-    const size_t row = (size_t)(vy < 0 ? N + vy : vy);
-    const size_t slab = (size_t)(vz < 0 ? N + vz : vz);
-    const size_t di = (size_t)vx * 2 + row * nxf + slab * nxf * (size_t)N;
-    const size_t ni = (size_t)vx + row * (size_t)w2 + slab * (size_t)w2 * (size_t)N;
-    if (v.w != 0.f) {
-      atomicAdd(&J.data[di], v.x);
-      J.data[di + 1] = 0.0f;
-    } else {
-      atomicAdd(reinterpret_cast<float2 *>(&J.data[di]), make_float2(v.x, v.y));
-    }
-    if (v.z != 0.f) atomicAdd(&J.norm[ni], v.z);
-  }
-  __syncthreads();
-}
-
-
-// ------------------------------------------------------------------ v4
+// ------------------------------------------------------------------ pixels
 // Pixel-major variant for the windows one or two taps wide (nearest,
 // gauss_2, trilinear), where walking columns spends most of its
 // instructions finding candidate pixels for two taps.  Each warp takes
@@ -792,13 +397,12 @@ struct Smem4 {
 constexpr int kRexpEntries = 376;
 constexpr int kRexpCopies = 8;
 
-// Util::fast_exp(f) for f in [-19.98, 0] read from the interleaved copies.
-// The index (int)(-f*50.0+0.5) is formed in double as the reference forms it:
-// -f*50 + 0.5 is exact in double, so one DFMA and a truncating conversion give
-// it (1 % faster here than an exact FP32 construction of the same index).
-__device__ __forceinline__ float rexp_lookup(float f, const float *rexp) {
-  const int g = __double2int_rz(__fma_rn((double)(-f), 50.0, 0.5));
-  return rexp[g * kRexpCopies + (threadIdx.x & (kRexpCopies - 1))];
+// Util::fast_exp(-y) for y in [0, 7.5) read from the interleaved copies.  The
+// reference's index (int)(y*50.0+0.5) is floor(50y + 1/2): one multiply-add
+// rounded down onto a spacing of 1/4 leaves it in mantissa bits 2 and up.
+__device__ __forceinline__ float rexp_lookup(float y, const float *rexp) {
+  const int t = __float_as_int(__fmaf_rd(y, 50.0f, 2097152.5f)) & 0x1FFC;
+  return rexp[t * (kRexpCopies / 4) + (threadIdx.x & (kRexpCopies - 1))];
 }
 
 // Slot of local cell (lx, ly, lz) in the component arrays.  Each pair of rows
@@ -939,25 +543,50 @@ __device__ __forceinline__ void pixel_pass(const InsertJob &J, const Smem4 &S, c
           dyy[q] = __fmul_rn(dy, dy);
           dzz[q] = __fmul_rn(dz, dz);
         }
+        float wt[8], tre = val.x, tim = val.y;   // the weights, and what they multiply
 #pragma unroll
-        for (int c = 0; c < 2; c++)
+        for (int t = 0; t < 8; t++) {
+          const int a = t & 1, b = (t >> 1) & 1, c = t >> 2;
+          if (MODE == MODE_GAUSS2) {
+            const float r = __fadd_rn(__fadd_rn(dxx[a], dyy[b]), dzz[c]);
+            wt[t] = __fmul_rn(rexp_lookup(__fmul_rn(r, h), S.rexp), w);
+          } else {
+            float vre, vim;
+            tap_value<MODE>(x0 + a, y0 + b, z0 + c, xx, yy, zz, val.x, val.y, w, h, nullptr, vre,
+                            vim, wt[t]);
+          }
+        }
+        if (base[0] == 0) {   // tiles with x = 0 cells: their placement rules
 #pragma unroll
-          for (int b = 0; b < 2; b++)
+          for (int t = 0; t < 8; t++)
+            tile_tap(S, sg, x0 + (t & 1), y0 + ((t >> 1) & 1), z0 + (t >> 2), base, ext,
+                     __fmul_rn(tre, wt[t]), __fmul_rn(tim, wt[t]), wt[t]);
+          continue;
+        }
+        // the window's cells in the tile (mirrored in the conjugate pass),
+        // their bounds tested once per axis
+        if (sg < 0) tim = -tim;
+        int lx[2], ly[2], lz[2];
+        bool ix[2], iy[2], iz[2];
 #pragma unroll
-            for (int a = 0; a < 2; a++) {
-              float vre, vim, vw;
-              if (MODE == MODE_GAUSS2) {
-                const float r = __fadd_rn(__fadd_rn(dxx[a], dyy[b]), dzz[c]);
-                const float gg = __fmul_rn(rexp_lookup(__fmul_rn(-r, h), S.rexp), w);
-                vre = __fmul_rn(val.x, gg);
-                vim = __fmul_rn(val.y, gg);
-                vw = gg;
-              } else {
-                tap_value<MODE>(x0 + a, y0 + b, z0 + c, xx, yy, zz, val.x, val.y, w, h, nullptr,
-                                vre, vim, vw);
-              }
-              tile_tap(S, sg, x0 + a, y0 + b, z0 + c, base, ext, vre, vim, vw);
-            }
+        for (int q = 0; q < 2; q++) {
+          lx[q] = sg * (x0 + q) - base[0];
+          ly[q] = sg * (y0 + q) - base[1];
+          lz[q] = sg * (z0 + q) - base[2];
+          ix[q] = (unsigned)lx[q] <= (unsigned)(ext[0] - base[0]);
+          iy[q] = (unsigned)ly[q] <= (unsigned)(ext[1] - base[1]);
+          iz[q] = (unsigned)lz[q] <= (unsigned)(ext[2] - base[2]);
+        }
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const int a = t & 1, b = (t >> 1) & 1, c = t >> 2;
+          if (ix[a] && iy[b] && iz[c]) {
+            const int s = cell_slot(lx[a], ly[b], lz[c]);
+            atomicAdd(&S.are[s], __fmul_rn(tre, wt[t]));
+            atomicAdd(&S.aim[s], __fmul_rn(tim, wt[t]));
+            atomicAdd(&S.awt[s], wt[t]);
+          }
+        }
       }
     }
     __syncwarp();
@@ -1111,71 +740,6 @@ __global__ void __launch_bounds__(col::NT, 2)
         if (threadIdx.x == 0) atomicOr(err, 4);
     }
   }
-}
-
-__global__ void __launch_bounds__(col::NT, 3)
-    k_column3(const InsertJob *__restrict__ jobs, const int4 *__restrict__ work, int nwork,
-              int block, int *counter, const float *__restrict__ exp_g, float h2, float h5,
-              ExpSteps st2, ExpSteps st5, int maxN, int *err) {
-  extern __shared__ float4 s_dyn[];
-  __shared__ int s_work;
-  __shared__ int s_wcount[col::NT / 32];
-  __shared__ int s_gcount[3];
-  __shared__ int s_state[2];
-  col::Smem3 S;
-  S.acc = s_dyn;
-  S.steps = nullptr;
-  S.exp = reinterpret_cast<float *>(s_dyn + col::NV);
-  S.rtab = S.exp + 1000;
-  S.xmax = reinterpret_cast<short *>(S.rtab + maxN + 2);
-  S.hits = reinterpret_cast<unsigned short *>(S.xmax + maxN + 2);
-  S.tmp = S.hits + block;
-  S.wcount = s_wcount;
-  S.gcount = s_gcount;
-  S.state = s_state;
-  for (int i = threadIdx.x; i < 1000; i += blockDim.x) S.exp[i] = exp_g[i];
-  if (threadIdx.x == 0) { s_state[0] = -1; s_state[1] = -1; }
-  while (true) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_work = atomicAdd(counter, 1);
-    __syncthreads();
-    const int wi = s_work;
-    if (wi >= nwork) break;
-    const int4 wk = work[wi];
-    const InsertJob J = jobs[wk.x];
-    const int s0 = wk.z, s1 = min(min(wk.w, wk.z + block), J.np * J.nsym);
-    switch (J.mode) {
-      case MODE_GAUSS2: col::tile_item3<MODE_GAUSS2>(J, wk.y, s0, s1, S, h2, st2, err); break;
-      case MODE_GAUSS5: col::tile_item3<MODE_GAUSS5>(J, wk.y, s0, s1, S, h5, st5, err); break;
-      case MODE_NEAREST: col::tile_item3<MODE_NEAREST>(J, wk.y, s0, s1, S, h2, st2, err); break;
-      case MODE_TRILINEAR: col::tile_item3<MODE_TRILINEAR>(J, wk.y, s0, s1, S, h2, st2, err); break;
-      default:
-        if (threadIdx.x == 0) atomicOr(err, 4);
-    }
-  }
-}
-
-cudaError_t launch_column3(const InsertJob *d_jobs, const int4 *d_work, int nwork, int block,
-                           int *d_counter, int maxN, cudaStream_t st) {
-  if (nwork == 0) return cudaSuccess;
-  const Consts &c = consts();
-  const size_t smem = sizeof(float4) * col::NV + sizeof(float) * 1000 +
-                      sizeof(float) * (maxN + 2) + sizeof(short) * (maxN + 2) +
-                      2 * sizeof(unsigned short) * block;
-  cudaError_t ea = set_max_smem((const void *)k_column3, smem);
-  if (ea != cudaSuccess) return ea;
-  cudaError_t e = zero_counter(d_counter, st);
-  if (e != cudaSuccess) return e;
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_column3, col::NT, smem);
-  if (per_sm < 1) per_sm = 1;
-  const int grid = std::max(1, std::min(nwork, sms * per_sm));
-  note_launch();
-  k_column3<<<grid, col::NT, smem, st>>>(d_jobs, d_work, nwork, block, d_counter, c.d_exp, c.h2,
-                                         c.h5, c.steps2, c.steps5, maxN, c.d_err);
-  return cudaGetLastError();
 }
 
 __global__ void __launch_bounds__(col::NT, 3)

@@ -61,6 +61,28 @@ struct DevBuf {
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
+// Workspaces the plane kernel inserts into and its merges clear again (a
+// partial volume; copies of the cells near the origin): zero between launches,
+// whatever sizes shared them.  Without memory for them the insertion goes
+// straight to the accumulators.
+struct ZeroBuf : DevBuf {
+  // Whether the buffer holds at least `bytes`, zeroed on st when it grew.
+  bool ensure_zero(size_t bytes, cudaStream_t st) {
+    if (bytes <= cap) return true;
+    if (ensure(bytes) == FR_OK && cudaMemsetAsync(p, 0, cap, st) == cudaSuccess) return true;
+    cudaGetLastError();
+    release();
+    return false;
+  }
+};
+struct PlaneBufs {
+  ZeroBuf data, norm, centre;
+  // Makes room for a call (plane_partial, plane_centre decide what it uses).
+  void ensure(int N, long slices, cudaStream_t st);
+  void release() {
+    for (DevBuf *b : {(DevBuf *)&data, (DevBuf *)&norm, (DevBuf *)&centre}) b->release();
+  }
+};
 
 // Pinned host staging for per-call uploads (metadata blocks, job tables,
 // work lists).  A pageable source would make cudaMemcpyAsync wait for the
@@ -320,6 +342,7 @@ struct fr_recon {
   // scratch
   fr::DevBuf s_in, s_slices, s_rot, s_w, s_t3d, s_img, s_img2, s_spec, s_ctf, s_txy, s_out,
       s_ssnr, s_jobs, s_work, s_counter;
+  fr::PlaneBufs plane;
   fr::PlanCache plans;
   int tile = -1;              // gather tile shape (-1: tuned default)
   std::vector<int> tiles;
@@ -371,6 +394,10 @@ int stream_leave_all(const std::vector<fr_recon *> &rs, cudaStream_t st,
                      std::shared_ptr<SharedEvent> *reuse = nullptr);
 InsertJob make_job(fr_recon *r, const float2 *slices, const float *t3d, const float *pw, int np);
 int run_scatter(const InsertJob &j0, bool edge_only, cudaStream_t st);
+// The plane-column insertion of one job: through the partial volume in turns
+// of kPlaneTurn slices when the call is large enough (plane_partial), with
+// centre copies from 16 slices on, as far as `b` has room for them.
+int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st);
 int insert_device(fr_recon *r, const float2 *d_slices, const float *d_t3d, const float *d_pw, int np,
                   int schedule, const float *d_ssnr, int nssnr);
 int check_device_error(fr_recon *r);

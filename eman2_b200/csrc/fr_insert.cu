@@ -7,8 +7,9 @@
 //
 // Three kernels:
 //  * k_scatter  -- one thread per (slice, pixel); every tap is added with FP32
-//                  atomics exactly as add_complex_at_fast places it.  Used for
-//                  single slices and small batches.
+//                  atomics exactly as add_complex_at_fast places it: nearest,
+//                  the per-pixel weights and z sizes only it takes, and a few
+//                  small slices of the other modes (fr_plane.cu has the rest).
 //  * k_gather   -- a persistent kernel over voxel tiles.  A tile owns its
 //                  cells; for each slice whose plane passes the tile it stages
 //                  the slice's pixel patch in shared memory and every voxel
@@ -57,54 +58,6 @@ cudaError_t launch_compose(const float *d_arg, const float *d_sym, int np, int n
 }
 
 // ------------------------------------------------------------- scatter path
-// One pixel's full insert_pixel with atomics.  Window selection and reject
-// rules follow libEM/reconstructor_tools.cpp:113-126 (nearest),
-// :128-166 (gauss_2), :191-230 (trilinear), :315-376 (gauss_5).
-// face_only: process only taps with a coordinate at +-N/2 (edge kernel).
-// NZ: the volume's z size (its window clamps and placement; N when cubic).
-template <int MODE>
-__device__ __forceinline__ void insert_pixel_atomic(float *__restrict__ data, float *__restrict__ norm,
-                                                    int N, int NZ, float xx, float yy, float zz,
-                                                    float re, float im, float w, float h,
-                                                    const float *__restrict__ table, bool face_only) {
-  const int n2 = N >> 1, nz2 = NZ >> 1;
-  if (MODE == MODE_NEAREST) {
-    const int x0 = (int)floorf(__fadd_rn(xx, 0.5f));
-    const int y0 = (int)floorf(__fadd_rn(yy, 0.5f));
-    const int z0 = (int)floorf(__fadd_rn(zz, 0.5f));
-    if (face_only && abs(x0) != n2 && abs(y0) != n2 && abs(z0) != nz2) return;
-    add_tap_atomic(data, norm, N, NZ, x0, y0, z0, __fmul_rn(re, w), __fmul_rn(im, w), w);
-  } else if (MODE == MODE_GAUSS2 || MODE == MODE_TRILINEAR) {
-    const int x0 = (int)floorf(xx), y0 = (int)floorf(yy), z0 = (int)floorf(zz);
-    if (x0 < -n2 - 1 || y0 < -n2 - 1 || z0 < -nz2 - 1 || x0 > n2 || y0 > n2 || z0 > nz2) return;
-    for (int k = z0; k <= z0 + 1; k++)
-      for (int j = y0; j <= y0 + 1; j++)
-        for (int i = x0; i <= x0 + 1; i++) {
-          if (face_only && abs(i) != n2 && abs(j) != n2 && abs(k) != nz2) continue;
-          float vre, vim, vw;
-          tap_value<MODE>(i, j, k, xx, yy, zz, re, im, w, h, table, vre, vim, vw);
-          add_tap_atomic(data, norm, N, NZ, i, j, k, vre, vim, vw);
-        }
-  } else {  // MODE_GAUSS5
-    int x0 = floor_minus_2p5(xx), y0 = floor_minus_2p5(yy), z0 = floor_minus_2p5(zz);
-    if (x0 < -n2 - 4 || y0 < -n2 - 4 || z0 < -nz2 - 4 || x0 > n2 + 3 || y0 > n2 + 3 ||
-        z0 > nz2 + 3)
-      return;
-    int x1 = x0 + 5, y1 = y0 + 5, z1 = z0 + 5;
-    x0 = max(x0, -n2); x1 = min(x1, n2);
-    y0 = max(y0, -n2); y1 = min(y1, n2);
-    z0 = max(z0, -nz2); z1 = min(z1, nz2);
-    for (int k = z0; k <= z1; k++)
-      for (int j = y0; j <= y1; j++)
-        for (int i = x0; i <= x1; i++) {
-          if (face_only && abs(i) != n2 && abs(j) != n2 && abs(k) != nz2) continue;
-          float vre, vim, vw;
-          tap_value<MODE>(i, j, k, xx, yy, zz, re, im, w, h, table, vre, vim, vw);
-          add_tap_atomic(data, norm, N, NZ, i, j, k, vre, vim, vw);
-        }
-  }
-}
-
 // EMData::get_complex_at(x, y, z) of a complex volume [N][N][N+2]
 // (libEM/emdata_core.cpp:134-144): 0 outside, the conjugate for x < 0.
 __device__ __forceinline__ float2 volume_at(const float *__restrict__ v, int N, int x, int y, int z) {

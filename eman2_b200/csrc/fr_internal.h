@@ -37,6 +37,7 @@ extern const TileShape kTiles[kNumTiles];
 struct InsertJob {
   float *data;               // [N][N][N+2]
   float *norm;               // [N][N][N/2+1]
+  float *fdata, *fnorm;      // the accumulators, where data and norm are a partial volume
   const float2 *slices;      // [np][N][N/2+1]
   const float *t3d;          // [np*nsym][9]
   const float *pw;           // [np] weight per particle
@@ -54,6 +55,11 @@ struct InsertJob {
   int N, mode, nsym, np;
   int tiles_x, tiles_y, tiles_z;
   int nz;                    // the volume's z size when it differs from N (scatter only); 0: N
+  int corners;               // the pixels fill the square, not the disk
+  // copies of the cells within `centre` of the origin, [copies] values then
+  // [copies] weights, or null (fr_plane.cu); slice s adds to copy s % copies
+  float *cdata;
+  int centre, copies;
 };
 
 // Launch accounting (fr_api.cu).
@@ -101,7 +107,7 @@ cudaError_t launch_scatter_tables(const InsertJob &j, const float *table, float 
 // (or rim) count of those jobs.
 cudaError_t launch_scatter_multi(const InsertJob *d_jobs, const int2 *d_units, int nunits,
                                  int max_px, bool edge_only, cudaStream_t st);
-// Column-owner kernel (fr_column.cu): 16^3 tiles, work items (job, tile,
+// Staged column-owner kernel (fr_column.cu): 16^3 tiles, work items (job, tile,
 // first slice, end slice) over slice blocks of at most kColumnBlock.
 constexpr int kColumnTile = kNumTiles;   // tile id selecting the column kernel
 constexpr int kColumnBlock = 1024;       // largest slice block (shared-memory hit list)
@@ -128,22 +134,67 @@ cudaError_t launch_column(const InsertJob *d_jobs, const int4 *d_work, int nwork
                           int *d_counter, int max_mode, cudaStream_t st);
 void column_tiles(int N, int mode, int corners, std::vector<int> &out, int &tx, int &ty, int &tz,
                   std::vector<float> *dist = nullptr);
-// The barrier-free column kernel (no patch staging; hits grouped by axis).
-constexpr int kColumn3Tile = kNumTiles + 1;
-// The pixel-major kernel for windows one or two taps wide (nearest,
-// gauss_2, trilinear); gauss_5 jobs given this id take k_column3.
+// The plane-column kernel (fr_plane.cu): gauss_5, and gauss_2 and trilinear up
+// to the size effective_tile states; of all three, every call of the scatter
+// schedule.
+constexpr int kPlaneTile = kNumTiles + 1;
+// The pixel-major kernel: nearest_neighbor, and gauss_2 and trilinear beyond
+// that size.
 constexpr int kPixelTile = kNumTiles + 2;
+inline bool plane_mode(int mode) { return mode == 2 || mode == 5 || mode == 6; }
+cudaError_t launch_plane(const InsertJob &j, cudaStream_t st);
+// The same with caller-supplied exp table and Gaussian factor.
+cudaError_t launch_plane_tables(const InsertJob &j, const float *table, float h, cudaStream_t st);
+// Several jobs of one mode in one launch: segment i's job has `parts` units
+// per slice, numbered from `first` on.  plane_seg fills a segment and returns
+// the next first unit (-1: more units than an int holds).
+struct PlaneSeg {
+  int job, first, parts;
+};
+int plane_seg(const InsertJob &j, int job, int first, PlaneSeg &out);
+cudaError_t launch_plane_multi(const InsertJob *d_jobs, const PlaneSeg *d_segs, int nsegs,
+                               int units, int mode, int maxN, cudaStream_t st);
+// A few small slices of the two-tap windows: one thread per pixel ends sooner
+// than one lane per column, which walks 5 to 6 pixels and their rows (gauss_2,
+// c1: N = 192 6.7 against 10.6 us, N = 384 10.8 against 13.6; with c4 24.7
+// against 29.3; with d7 68 against 58).  gauss_5 has none (N = 48, c1: 72
+// against 44 us).
+inline bool plane_small(int mode, int N, long slices) {
+  return mode != 5 && slices < 64 && slices * N * N < 1000000;
+}
+// A volume cell gets one addition per slice that reaches it.  Calls of this
+// many slices or more insert into a partial volume in turns of kPlaneTurn
+// slices, each added to the accumulators once (launch_merge, which clears the
+// partial volume again), so a cell's sums stay short ones however many
+// slices a job has.  The merge costs as much as about N / 4 slices' insertion,
+// whence the limit.
+constexpr int kPlaneTurn = 2048;
+inline bool plane_partial(int N, long slices) { return slices >= 256 && slices * 3 >= 8L * N; }
+// Every slice meets the cells near the origin.  Calls of 16 slices or more
+// add them to one of several copies of that cube, about 64 slices to each,
+// summed in double afterwards (launch_merge_centre, which clears them), so
+// those sums stay as short as the others.  Returns the copies' bytes (0:
+// none), their half-width and number.
+size_t plane_centre(int N, long slices, int &half, int &copies);
+// One job (one) or every job of this mode in a device table (those without
+// copies return; another mode's may still be inserting on another stream).
+cudaError_t launch_merge_centre(const InsertJob *d_jobs, int njobs, const InsertJob *one, int mode,
+                                int half, cudaStream_t st);
+cudaError_t launch_merge(float *data, float *norm, float *pdata, float *pnorm, int N, int corners,
+                         cudaStream_t st);
 cudaError_t launch_pixel(const InsertJob *d_jobs, const int4 *d_work, int nwork, int block,
                          int *d_counter, int maxN, cudaStream_t st);
-// The kernel a job of this mode runs for a requested tile id.
-inline int effective_tile(int tile, int mode) {
-  return (tile == kPixelTile && mode == 5 /* gauss_5 */) ? kColumn3Tile : tile;
+// The kernel a job of this mode and size runs for a requested tile id.  The
+// two-tap windows' runs are short, so beyond the L2 cache the plane-column
+// kernel waits for memory on every run, while the tile kernel adds to a tile
+// many times before it flushes it: N = 288 21.6 against 26.2 us a particle
+// (gauss_2, d7), N = 384 47.6 against 45.9, N = 480 87 against 72.
+inline int effective_tile(int tile, int mode, int N) {
+  if (tile != kPlaneTile && tile != kPixelTile) return tile;
+  return mode == 5 || (plane_mode(mode) && N <= 352) ? kPlaneTile : kPixelTile;
 }
-inline bool is_column_tile(int tile) {
-  return tile == kColumnTile || tile == kColumn3Tile || tile == kPixelTile;
-}
-cudaError_t launch_column3(const InsertJob *d_jobs, const int4 *d_work, int nwork, int block,
-                           int *d_counter, int maxN, cudaStream_t st);
+// The kernels over 16^3 tiles and slice blocks (int4 work items).
+inline bool is_column_tile(int tile) { return tile == kColumnTile || tile == kPixelTile; }
 // Ordered work list (tile ids of a job that can receive interior taps).
 void gather_tiles(int N, int mode, int tile, int corners, std::vector<int> &out, int &tx, int &ty,
                   int &tz);

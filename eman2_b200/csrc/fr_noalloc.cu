@@ -148,6 +148,8 @@ extern "C" int fr_insert_slices_noalloc(const float *d_slices, int n, int N, int
   memset(&j, 0, sizeof j);
   j.data = d_data;
   j.norm = d_norm;
+  j.fdata = d_data;
+  j.fnorm = d_norm;
   j.slices = reinterpret_cast<const float2 *>(d_slices);
   j.t3d = scr + kT3dOff;
   j.pw = d_weights;
@@ -162,6 +164,7 @@ extern "C" int fr_insert_slices_noalloc(const float *d_slices, int n, int N, int
   volatile float i2g = (float)(4.0 / (M_PI * M_PI));
   volatile float i5g = (float)(10.4 / (M_PI * M_PI));
   const float h = mode == FR_MODE_GAUSS5 ? 1.0f / i5g : 1.0f / i2g;
-  CU(launch_scatter_tables(j, scr + kExpOff, h, st));
+  CU(plane_mode(mode) ? launch_plane_tables(j, scr + kExpOff, h, st)
+                      : launch_scatter_tables(j, scr + kExpOff, h, st));
   return FR_OK;
 }

@@ -1,0 +1,786 @@
+// fr_plane.cu -- the plane-column insertion kernel (gauss_2, gauss_5,
+// trilinear).
+//
+// A slice's taps lie in a slab around its plane.  With A the axis along which
+// the plane's normal is largest, B and C the other two, every tap column
+// (b, c) crosses that slab in one short run of cells along A (at most 7 cells
+// for the two-tap windows, 19 for gauss_5).  One lane owns one column of one
+// slice: it walks the pixels whose window covers the column, sums their taps
+// into the run, held in its own shared-memory words (gauss_5 keeps the six
+// cells of the current window in registers), and at the end adds the run's
+// sums to the volume, one reduction per touched cell, under the placement
+// rules of add_complex_at_fast.  No lane ever shares a cell with another
+// before that, so there are neither barriers nor shared-memory atomics, and a
+// warp (an 8 x 4 patch of columns) depends on no other warp.
+//
+// What bounds it: issue slots (76 % of cycles issue at gauss_5, 75 % at
+// gauss_2 while the volume fits L2), at 69 % of lanes busy: the windows of a
+// warp's columns hold unequal pixel counts.  A gauss_5 tap takes 36 thread
+// instructions, 64 in the tile columns: a pixel's coordinates and window serve
+// six taps, the weights go through packed operations, and a cell leaves the
+// registers once.
+// Measured on one B200, insertion alone (the kernels it took over from in
+// parentheses): gauss_5, d7, N = 384, 64 particles 21.3 ms (46.8, tile columns
+// with shared read-modify-writes), one particle 0.43 ms (1.32, an atomic per
+// tap); gauss_2, c1, N = 192, 2048 particles 1.42 ms (2.12, tiles with shared
+// atomics).  Shared memory: three blocks of eight warps fit an SM at gauss_5's
+// 72 KB and 80 registers; more blocks at fewer registers spilled (gauss_2 at 4
+// and 5 blocks: 1.60 and 1.71 ms).
+//
+// Tap selection and weights are the reference's bit for bit (window start,
+// exp-table index, radius); a cell's taps of one slice are summed before they
+// reach the volume, so only the order of additions differs from one atomic
+// per tap.
+//
+// Reference: do_insert_slice_work (libEM/reconstructor.cpp:1122-1210),
+// insert_pixel (libEM/reconstructor_tools.cpp:128-230, 315-376),
+// add_complex_at_fast (libEM/emdata_core.h:368-410).
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <map>
+#include <mutex>
+#include <tuple>
+
+#include "fr_device.cuh"
+#include "fr_internal.h"
+
+namespace fr {
+namespace plane {
+
+constexpr int NT = 256;         // threads: 8 independent warps
+constexpr int NW = NT / 32;
+constexpr float kDel = 0.02f;   // slack on the approximate plane geometry
+
+// Taps of a window along one axis, its reach (a pixel at p covers tap t iff
+// t - lo <= p < t + hi) and the most cells a column's run can hold: the
+// plane's height over the (lo+hi)-wide square window varies by at most
+// 2 (lo+hi), its slopes being at most 1 along the dominant axis.  EXP: the
+// fast_exp entries kept in shared memory; gauss_5's largest r*h*50 is
+// 36.75 * 0.949 * 50 < 1745, past the reference's 1000 entries (the rest read
+// as 0 and are replaced), gauss_2's 3 * 2.468 * 50 < 371.
+template <int MODE> struct Win;
+template <> struct Win<MODE_GAUSS5> {
+  static constexpr float lo = 2.5f, hi = 3.5f;
+  static constexpr int K = 6, W = 20, CTAS = 3, EXP = 2048;
+};
+template <> struct Win<MODE_GAUSS2> {
+  static constexpr float lo = 1.0f, hi = 1.0f;
+  static constexpr int K = 2, W = 8, CTAS = 3, EXP = 512;
+};
+template <> struct Win<MODE_TRILINEAR> : Win<MODE_GAUSS2> {
+  static constexpr int EXP = 0;
+};
+
+// What a warp's columns of one slice share, in the warp's own shared words.
+// u*, v*: the first two rows of the rotation, components along A, B and C.
+// The rest is linear in the column (tb, tc): the rows its window meets
+// (ylo, yhi), the first cells its pixels can start at (alo, ahi), and per row
+// y the x range [lo, hi] each of its two window constraints leaves, lo = L +
+// tb * I + y * S and hi likewise from U (kDel wider than the window).
+struct SliceGeom {
+  float ua, ub, uc, w;
+  float va, vb, vc, pad;
+  float yb, yc, ylo, yhi;
+  float ab, ac, alo, ahi;
+  float Ib, Lb, Ub, Sb;
+  float Ic, Lc, Uc, Sc;
+};
+
+struct Smem {
+  const float *exp;     // [Win<MODE>::EXP]
+  const float *rtab;    // [N+2]
+  const short *xmax;    // [N]
+  SliceGeom *geom;      // this warp's
+  float2 *sv;           // [W][32] this warp's value sums, lane-minor
+  float *sw;            // [W][32] this warp's weight sums
+};
+
+// Util::fast_exp's table entry for f = -y, y in [0, 41).  The reference's
+// index (int)(y*50.0 + 0.5) (double) is floor(50y + 1/2): one multiply-add
+// rounded down onto the spacing of [2^21, 2^22), 1/4, leaves four times that
+// floor (and two lower bits) in the mantissa, which is the entry's byte
+// offset.  Exact for every float y: the product and sum are not rounded before.
+constexpr float kIndex = 2097152.5f;   // 2^21 + 1/2
+__device__ __forceinline__ float exp_at(float t, const float *tab) {
+  return *reinterpret_cast<const float *>(reinterpret_cast<const char *>(tab) +
+                                          (__float_as_int(t) & 0x1FFC));
+}
+
+// First tap of a pixel's window, as an integer-valued float: floor(p - 2.5)
+// (gauss_5) or floor(p), by additions rounded down onto a spacing of 1/2 and
+// then 1 (floor of a floor onto a finer grid), |p| < 2^20.
+template <int MODE> __device__ __forceinline__ float win_start(float p, int &start) {
+  float t;
+  if (MODE == MODE_GAUSS5) t = __fadd_rd(__fadd_rd(p, 6291456.0f - 2.5f), 6291456.0f);
+  else t = __fadd_rd(p, 12582912.0f);
+  start = __float_as_int(t) - 0x4B400000;
+  return __fsub_rn(t, 12582912.0f);
+}
+
+// Pairs of floats: one issue slot for two operations, each rounded as its
+// scalar form.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack(f2 v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// The squares of a pair, each rounded before it is added to: a packed product
+// whose only use is a packed sum comes out of the assembler as one fused
+// operation, .rn or not, so these two stay scalar.
+__device__ __forceinline__ f2 square2(f2 v) {
+  float a, b;
+  unpack(v, a, b);
+  return pack(__fmul_rn(a, a), __fmul_rn(b, b));
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 fma2_rd(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Adds (re, im, w) to one cell of the run.
+__device__ __forceinline__ void cell_add(const Smem &S, int at, float re, float im, float w) {
+  float2 v = S.sv[at];
+  v.x += re;
+  v.y += im;
+  S.sv[at] = v;
+  S.sw[at] += w;
+}
+
+// Word of cell (i, j, l), i >= 0, in a centre copy of half-width c.
+__device__ __forceinline__ int centre_cell(int c, int i, int j, int l) {
+  return ((l + c) * (2 * c + 1) + j + c) * (c + 1) + i;
+}
+
+// Adds the sums of tap cell (i, j, l) of a slice to the volume, or to the
+// slice's copy of the cells near the origin (see plane_centre).
+__device__ __forceinline__ void place(const InsertJob &J, float2 *cd, float *cn, int i, int j, int l,
+                                      float re, float im, float w) {
+  const int N = J.N, n2 = N >> 1, w2 = n2 + 1;
+  const int ia = abs(i), c = J.centre;
+  const bool near = cd && ia <= c && abs(j) <= c && abs(l) <= c;
+  if (ia == 0 || ia >= n2) {
+    if (near) {   // i = 0 (c < N/2): both mirror cells, the mirrored one without weight
+      const int at = centre_cell(c, 0, j, l);
+      const bool origin = j == 0 && l == 0;
+      if (!origin) atomicAdd(cd + centre_cell(c, 0, -j, -l), make_float2(re, -im));
+      atomicAdd(cd + at, make_float2(re, origin ? 0.0f : im));
+      atomicAdd(cn + at, w);
+    } else {
+      add_tap_atomic(J.data, J.norm, N, N, i, j, l, re, im, w);
+    }
+    return;
+  }
+  if (abs(j) > n2 || abs(l) > n2) return;
+  // add_complex_at_fast away from the planes x = 0 and |x| = N/2: the cell,
+  // or for x < 0 its mirror, conjugated
+  if (i < 0) {
+    j = -j;
+    l = -l;
+    im = -im;
+  }
+  size_t at;
+  float2 *data = reinterpret_cast<float2 *>(J.data);
+  float *norm = J.norm;
+  if (near) {
+    at = centre_cell(c, ia, j, l);
+    data = cd;
+    norm = cn;
+  } else {
+    at = (size_t)ia + (size_t)((j < 0 ? N + j : j) + (l < 0 ? N + l : l) * N) * w2;
+  }
+  atomicAdd(data + at, make_float2(re, im));
+  atomicAdd(norm + at, w);
+}
+
+// One column (tb, tc) of the slice, a lane each.
+template <int MODE>
+__device__ __forceinline__ void column(const InsertJob &J, const Smem &S, int A, int tb, int tc,
+                                       const float2 *__restrict__ sl, float h, float2 *cd,
+                                       float *cn) {
+  constexpr float LO = Win<MODE>::lo, HI = Win<MODE>::hi;
+  const int N = J.N, n2 = N >> 1, w2 = n2 + 1;
+  const int lane = threadIdx.x & 31;
+  const float Nf = (float)N;
+  const SliceGeom &G = *S.geom;
+  const float tbf = (float)tb, tcf = (float)tc;
+  // exact window bounds on the pixel's coordinates.  A gauss_5 pixel is
+  // skipped whole when its window starts below -N/2-4
+  // (libEM/reconstructor_tools.cpp:321), which only a column at -N/2 can meet.
+  const float edge = (float)(-n2) - 1.5f;
+  const float lob = MODE == MODE_GAUSS5 ? fmaxf(tbf - LO, edge) : tbf - LO, hib = tbf + HI;
+  const float loc = MODE == MODE_GAUSS5 ? fmaxf(tcf - LO, edge) : tcf - LO, hic = tcf + HI;
+  const float yv0 = fmaf(tbf, G.yb, tcf * G.yc), av0 = fmaf(tbf, G.ab, tcf * G.ac);
+  const int r0 = max(-n2, __float2int_ru(yv0 + G.ylo)),
+            r1 = min(n2 - 1, __float2int_rd(yv0 + G.yhi));
+  const int kb = __float2int_rd(av0 + G.alo);
+  const int nq = __float2int_rd(av0 + G.ahi) + Win<MODE>::K - kb;   // cells of the run
+  const float Lb = fmaf(tbf, G.Ib, G.Lb), Ub = fmaf(tbf, G.Ib, G.Ub);
+  const float Lc = fmaf(tcf, G.Ic, G.Lc), Uc = fmaf(tcf, G.Ic, G.Uc);
+  const float Sb = G.Sb, Sc = G.Sc;
+  const float ua = G.ua, ub = G.ub, uc = G.uc, w = G.w;
+  const float vscale = MODE == MODE_TRILINEAR ? 1.0f : w;
+  const int cell0 = lane - kb * 32;      // cell k of the run is word cell0 + 32 k
+
+#pragma unroll 1
+  for (int y = r0; y <= r1; y++) {
+    const float yf = (float)y;
+    const int xm = S.xmax[y + n2];
+    const float xlo = fmaxf(fmaxf(fmaf(yf, Sb, Lb), fmaf(yf, Sc, Lc)), 0.0f);
+    const float xhi = fminf(fminf(fmaf(yf, Sb, Ub), fmaf(yf, Sc, Uc)), (float)xm);
+    const int c0 = __float2int_ru(xlo), c1 = __float2int_rd(xhi);
+    if (c0 > c1) continue;
+    const float ry = S.rtab[y + n2];
+    const float qa = __fmul_rn(ry, G.va), qb = __fmul_rn(ry, G.vb), qc = __fmul_rn(ry, G.vc);
+    const float2 *rowp = sl + (size_t)(y < 0 ? N + y : y) * w2;
+    // heights rise along the walk, so gauss_5's window only moves up
+    const int dx = ua < 0.0f ? -1 : 1;
+    int x = ua < 0.0f ? c1 : c0;
+    float ar[6], ai[6], aw[6];
+    int cur = INT_MAX;     // gauss_5: the cell of ar[0], ...
+    if (MODE == MODE_GAUSS5) {
+#pragma unroll
+      for (int t = 0; t < 6; t++) ar[t] = ai[t] = aw[t] = 0.0f;
+    }
+#pragma unroll 1
+    for (int cnt = c1 - c0; cnt >= 0; cnt--, x += dx) {
+      const float rx = S.rtab[x + n2];
+      const float pb = __fmul_rn(__fadd_rn(__fmul_rn(rx, ub), qb), Nf);
+      const float pc = __fmul_rn(__fadd_rn(__fmul_rn(rx, uc), qc), Nf);
+      const float pa = __fmul_rn(__fadd_rn(__fmul_rn(rx, ua), qa), Nf);
+      bool in;
+      if (MODE == MODE_GAUSS5)
+        in = lob <= pb && pb < hib && loc <= pc && pc < hic && pa >= edge;
+      else
+        in = lob <= pb && pb < hib && loc <= pc && pc < hic;
+      if (!in) continue;
+      float2 v = __ldg(rowp + x);
+      if (x == 0 && y < 0) {   // reads (0, -y) conjugated
+        v = __ldg(sl + (size_t)(-y) * w2);
+        v.y = -v.y;
+      }
+      v.x *= vscale;
+      v.y *= vscale;
+      int a0;
+      const float a0f = win_start<MODE>(pa, a0);
+      const float db = __fsub_rn(tbf, pb), dc = __fsub_rn(tcf, pc);
+      if (MODE == MODE_TRILINEAR) {
+        // (libEM/reconstructor_tools.cpp:191-230): double products
+        const double ob = 1.0 - fabs((double)db), oc = 1.0 - fabs((double)dc);
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+          const double oa = 1.0 - fabs((double)__fsub_rn(a0f + (float)t, pa));
+          const double q = A == 2 ? (ob * oc) * oa : (oa * ob) * oc;
+          const float g = (float)(q * (double)w);
+          cell_add(S, cell0 + (a0 + t) * 32, v.x * g, v.y * g, g);
+        }
+        continue;
+      }
+      // r = (dx^2 + dy^2) + dz^2 (libEM/util.h:816-819): with A = z the sum
+      // of the other two comes first, else A's square is in the first sum
+      float f0 = __fmul_rn(db, db), f1 = __fmul_rn(dc, dc);
+      if (A == 2) {
+        f0 = __fadd_rn(f0, f1);
+        f1 = 0.0f;
+      }
+      const f2 npa = pack(-pa, -pa), f00 = pack(f0, f0), f11 = pack(f1, f1), hh = pack(h, h);
+      const f2 c50 = pack(50.0f, 50.0f), cidx = pack(kIndex, kIndex), aa = pack(a0f, a0f);
+      if (MODE == MODE_GAUSS2) {
+        const f2 d = add2(add2(aa, pack(0.0f, 1.0f)), npa);
+        const f2 r = add2(add2(square2(d), f00), f11);
+        float t0, t1;
+        unpack(fma2_rd(mul2(r, hh), c50, cidx), t0, t1);
+        const float g0 = exp_at(t0, S.exp), g1 = exp_at(t1, S.exp);   // r <= 3: in the table
+        const int at = cell0 + a0 * 32;
+        float2 q0 = S.sv[at], q1 = S.sv[at + 32];
+        float w0 = S.sw[at], w1 = S.sw[at + 32];
+        q0.x = fmaf(v.x, g0, q0.x);
+        q0.y = fmaf(v.y, g0, q0.y);
+        q1.x = fmaf(v.x, g1, q1.x);
+        q1.y = fmaf(v.y, g1, q1.y);
+        S.sv[at] = q0;
+        S.sv[at + 32] = q1;
+        S.sw[at] = w0 + g0;
+        S.sw[at + 32] = w1 + g1;
+        continue;
+      }
+      // gauss_5: move the window up to a0 (at most one cell: heights change
+      // by less than one a pixel), handing the cell below it over
+      cur = min(cur, a0);
+      if (cur < a0) {
+        cell_add(S, cell0 + cur * 32, ar[0], ai[0], aw[0]);
+#pragma unroll
+        for (int t = 0; t < 5; t++) { ar[t] = ar[t + 1]; ai[t] = ai[t + 1]; aw[t] = aw[t + 1]; }
+        ar[5] = ai[5] = aw[5] = 0.0f;
+        cur = a0;
+      }
+      float yv[6], g[6];
+#pragma unroll
+      for (int t = 0; t < 6; t += 2) {
+        const f2 d = add2(add2(aa, pack((float)t, (float)(t + 1))), npa);
+        const f2 r = add2(add2(square2(d), f00), f11);
+        const f2 yy = mul2(r, hh);
+        float t0, t1;
+        unpack(yy, yv[t], yv[t + 1]);
+        unpack(fma2_rd(yy, c50, cidx), t0, t1);
+        g[t] = exp_at(t0, S.exp);
+        g[t + 1] = exp_at(t1, S.exp);
+      }
+      // past the table (y > 19.98, r > 21.05) the reference calls exp: d^2 is
+      // at most 12.25 for the first tap and 6.25 for the others
+      const float f01 = f0 + f1;
+      if (f01 > 8.7f) {
+        if (yv[0] > 19.98f) g[0] = expf(-yv[0]);
+        if (f01 > 14.7f) {
+#pragma unroll
+          for (int t = 1; t < 6; t++)
+            if (yv[t] > 19.98f) g[t] = expf(-yv[t]);
+        }
+      }
+      const f2 vx = pack(v.x, v.x), vy = pack(v.y, v.y);
+#pragma unroll
+      for (int t = 0; t < 6; t += 2) {
+        const f2 gg = pack(g[t], g[t + 1]);
+        unpack(fma2(vx, gg, pack(ar[t], ar[t + 1])), ar[t], ar[t + 1]);
+        unpack(fma2(vy, gg, pack(ai[t], ai[t + 1])), ai[t], ai[t + 1]);
+        unpack(add2(gg, pack(aw[t], aw[t + 1])), aw[t], aw[t + 1]);
+      }
+    }
+    if (MODE == MODE_GAUSS5 && cur != INT_MAX) {
+#pragma unroll
+      for (int t = 0; t < 6; t++) cell_add(S, cell0 + (cur + t) * 32, ar[t], ai[t], aw[t]);
+    }
+  }
+  // the run into the volume; its words go back to zero for the next column
+  const float wscale = MODE == MODE_TRILINEAR ? 1.0f : w;
+#pragma unroll 1
+  for (int q = 0; q < nq; q++) {
+    const int at = q * 32 + lane;
+    const float2 v = S.sv[at];
+    const float s = S.sw[at];
+    if (v.x == 0.0f && v.y == 0.0f && s == 0.0f) continue;
+    S.sv[at] = make_float2(0.0f, 0.0f);
+    S.sw[at] = 0.0f;
+    const int k = kb + q;
+    const int i = A == 0 ? k : tb, j = A == 0 ? tb : (A == 1 ? k : tc), l = A == 2 ? k : tc;
+    place(J, cd, cn, i, j, l, v.x, v.y, s * wscale);
+  }
+}
+
+// x range lines of one window constraint t - lo <= x*u + y*v < t + hi.
+__device__ __forceinline__ void band(float lo, float hi, float u, float v, float &I, float &L,
+                                     float &U, float &S) {
+  if (fabsf(u) > 1e-4f) {
+    I = 1.0f / u;
+    const float p = (-lo - kDel) * I, q = (hi + kDel) * I;
+    L = fminf(p, q);
+    U = fmaxf(p, q);
+    S = -v * I;
+  } else {   // nearly constant along the row: left to the exact window test
+    I = S = 0.0f;
+    L = -1e9f;
+    U = 1e9f;
+  }
+}
+
+// Part `part` of `parts` of slice s: its patches, dealt to the warps.
+template <int MODE>
+__device__ __forceinline__ void slice_part(const InsertJob &J, const Smem &S, int s, int part,
+                                           int parts, float h, const float *__restrict__ table) {
+  constexpr float LO = Win<MODE>::lo, HI = Win<MODE>::hi;
+  const int N = J.N, n2 = N >> 1, w2 = n2 + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int p = s / J.nsym;
+  const float w = __ldg(&J.pw[p]);
+  if (w == 0.0f) return;
+  float M[6];
+#pragma unroll
+  for (int i = 0; i < 6; i++) M[i] = __ldg(&J.t3d[9 * (size_t)s + i]);
+  const float2 *sl = J.slices + (size_t)p * N * w2;
+  const float nx = M[1] * M[5] - M[2] * M[4], ny = M[2] * M[3] - M[0] * M[5],
+              nz = M[0] * M[4] - M[1] * M[3];
+  const float lu = M[0] * M[0] + M[1] * M[1] + M[2] * M[2];
+  const float lv = M[3] * M[3] + M[4] * M[4] + M[5] * M[5];
+  const float uv = M[0] * M[3] + M[1] * M[4] + M[2] * M[5];
+  if (!(fabsf(lu - 1.0f) < 0.01f && fabsf(lv - 1.0f) < 0.01f && fabsf(uv) < 0.01f)) {
+    // not a rotation (a caller's own matrix): tap by tap
+    for (int i = (part * NW + warp) * 32 + lane; i < N * w2; i += parts * NT) {
+      const int x = i % w2, y = i / w2 - n2;
+      if (x > S.xmax[y + n2]) continue;
+      float xx, yy, zz;
+      pixel_coords(S.rtab[x + n2], S.rtab[y + n2], M, (float)N, xx, yy, zz);
+      const float2 v = slice_value(sl, N, x, y);
+      insert_pixel_atomic<MODE>(J.fdata, J.fnorm, N, N, xx, yy, zz, v.x, v.y, w, h, table, false);
+    }
+    return;
+  }
+  const float ax = fabsf(nx), ay = fabsf(ny), az = fabsf(nz);
+  const int A = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
+  const float ua = A == 0 ? M[0] : (A == 1 ? M[1] : M[2]), ub = A == 0 ? M[1] : M[0],
+              uc = A == 2 ? M[1] : M[2];
+  const float va = A == 0 ? M[3] : (A == 1 ? M[4] : M[5]), vb = A == 0 ? M[4] : M[3],
+              vc = A == 2 ? M[4] : M[5];
+  const float idet = 1.0f / (ub * vc - uc * vb);
+  constexpr float E = 0.5f * (LO + HI) + kDel, C = 0.5f * (HI - LO);
+  constexpr float OFF = MODE == MODE_GAUSS5 ? 2.5f : 0.0f;
+  {
+    // (pb, pc) -> y and the plane's height pa, over the windows' extent
+    SliceGeom G;
+    G.ua = ua; G.ub = ub; G.uc = uc; G.w = w;
+    G.va = va; G.vb = vb; G.vc = vc; G.pad = 0.0f;
+    G.yb = -uc * idet;
+    G.yc = ub * idet;
+    const float y0 = C * (G.yb + G.yc), ey = E * (fabsf(G.yb) + fabsf(G.yc));
+    G.ylo = y0 - ey;
+    G.yhi = y0 + ey;
+    G.ab = (vc * ua - uc * va) * idet;
+    G.ac = (ub * va - vb * ua) * idet;
+    const float a0 = C * (G.ab + G.ac) - OFF, ea = E * (fabsf(G.ab) + fabsf(G.ac)) + kDel;
+    G.alo = a0 - ea;
+    G.ahi = a0 + ea;
+    band(LO, HI, ub, vb, G.Ib, G.Lb, G.Ub, G.Sb);
+    band(LO, HI, uc, vc, G.Ic, G.Lc, G.Uc, G.Sc);
+    __syncwarp();
+    if (lane == 0) *S.geom = G;
+    __syncwarp();
+  }
+  // tap columns the half disk x >= 0, |p| <= R reaches
+  const float R = J.corners ? n2 * 1.4143f + 1.0f : n2 + 0.52f;
+  const float hb = R * sqrtf(ub * ub + vb * vb), gb = R * fabsf(vb);
+  const float hc = R * sqrtf(uc * uc + vc * vc), gc = R * fabsf(vc);
+  const int b0 = max(-n2, __float2int_ru((ub < 0 ? -hb : -gb) - HI - kDel)),
+            b1 = min(n2, __float2int_rd((ub < 0 ? gb : hb) + LO + kDel));
+  const int c0 = max(-n2, __float2int_ru((uc < 0 ? -hc : -gc) - HI - kDel)),
+            c1 = min(n2, __float2int_rd((uc < 0 ? gc : hc) + LO + kDel));
+  if (b1 < b0 || c1 < c0) return;
+  float2 *cd = nullptr;
+  float *cn = nullptr;
+  if (J.cdata) {
+    const size_t cells = (size_t)(J.centre + 1) * (2 * J.centre + 1) * (2 * J.centre + 1);
+    cd = reinterpret_cast<float2 *>(J.cdata) + (s % J.copies) * cells;
+    cn = J.cdata + 2 * J.copies * cells + (s % J.copies) * cells;
+  }
+  const int nb = ((b1 - b0) >> 3) + 1, nc = ((c1 - c0) >> 2) + 1;
+  const float ex = (fabsf(vc) * (E + 3.5f) + fabsf(vb) * (E + 1.5f)) * fabsf(idet);
+  const float ey = (fabsf(ub) * (E + 1.5f) + fabsf(uc) * (E + 3.5f)) * fabsf(idet);
+  // patch q = qc * nb + qb, a stride of parts * NW patches at a time
+  const int first = part * NW + warp, stride = parts * NW;
+  const int dqc = stride / nb, dqb = stride - dqc * nb;
+  int qc = first / nb, qb = first - qc * nb;
+#pragma unroll 1
+  for (; qc < nc; qc += dqc, qb += dqb) {
+    if (qb >= nb) {
+      qb -= nb;
+      if (++qc >= nc) break;
+    }
+    const int tb0 = b0 + qb * 8, tc0 = c0 + qc * 4;
+    // the patch's windows in slice coordinates: any pixel of the half disk?
+    const float pb = tb0 + 3.5f + C, pc = tc0 + 1.5f + C;
+    const float xc = (pb * vc - pc * vb) * idet, yc = (ub * pc - uc * pb) * idet;
+    const float dx = fmaxf(0.0f, fabsf(xc) - ex), dy = fmaxf(0.0f, fabsf(yc) - ey);
+    if (xc + ex < -kDel || dx * dx + dy * dy > R * R) continue;
+    const int tb = tb0 + (lane & 7), tc = tc0 + (lane >> 3);
+    if (tb <= n2 && tc <= n2) column<MODE>(J, S, A, tb, tc, sl, h, cd, cn);
+    __syncwarp();
+  }
+}
+
+template <int MODE>
+__device__ __forceinline__ void smem_layout(Smem &S, unsigned char *dyn, int maxN, float *&exp,
+                                            float *&rtab, short *&xmax) {
+  constexpr int W = Win<MODE>::W;
+  const int warp = threadIdx.x >> 5;
+  S.geom = reinterpret_cast<SliceGeom *>(dyn) + warp;
+  float2 *sv = reinterpret_cast<float2 *>(dyn + NW * sizeof(SliceGeom));
+  float *sw = reinterpret_cast<float *>(sv + NW * W * 32);
+  exp = sw + NW * W * 32;
+  rtab = exp + Win<MODE>::EXP;
+  xmax = reinterpret_cast<short *>(rtab + maxN + 2);
+  S.sv = sv + warp * W * 32;
+  S.sw = sw + warp * W * 32;
+  S.exp = exp;
+  S.rtab = rtab;
+  S.xmax = xmax;
+}
+
+template <int MODE> size_t smem_bytes(int maxN) {
+  return NW * sizeof(SliceGeom) + (size_t)NW * Win<MODE>::W * 32 * 12 + Win<MODE>::EXP * 4 +
+         4 * (size_t)(maxN + 2) + 2 * (size_t)maxN;
+}
+
+template <int MODE>
+__device__ __forceinline__ void smem_init(const Smem &S, float *exp,
+                                          const float *__restrict__ table) {
+  for (int i = threadIdx.x; i < Win<MODE>::EXP; i += NT) exp[i] = i < 1000 ? __ldg(&table[i]) : 0.0f;
+  for (int i = threadIdx.x & 31; i < Win<MODE>::W * 32; i += 32) {
+    S.sv[i] = make_float2(0.0f, 0.0f);
+    S.sw[i] = 0.0f;
+  }
+}
+
+__device__ __forceinline__ void load_geometry(const InsertJob &J, float *rtab, short *xmax) {
+  for (int i = threadIdx.x; i < J.N + 2; i += NT) rtab[i] = __ldg(&J.rtab[i]);
+  for (int i = threadIdx.x; i < J.N; i += NT) xmax[i] = (short)__ldg(&J.xmax[i]);
+}
+
+}  // namespace plane
+
+// One job: unit u is part u % parts of slice u / parts.
+template <int MODE>
+__global__ void __launch_bounds__(plane::NT, plane::Win<MODE>::CTAS)
+    k_plane(InsertJob J, int units, int parts, float h, const float *__restrict__ table) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  plane::Smem S;
+  float *exp, *rtab;
+  short *xmax;
+  plane::smem_layout<MODE>(S, dyn, J.N, exp, rtab, xmax);
+  plane::smem_init<MODE>(S, exp, table);
+  plane::load_geometry(J, rtab, xmax);
+  __syncthreads();
+  for (int u = blockIdx.x; u < units; u += gridDim.x)
+    plane::slice_part<MODE>(J, S, u / parts, u % parts, parts, h, table);
+}
+
+// Several jobs of one mode: job segs[i].job has the units from segs[i].first on.
+template <int MODE>
+__global__ void __launch_bounds__(plane::NT, plane::Win<MODE>::CTAS)
+    k_plane_multi(const InsertJob *__restrict__ jobs, const PlaneSeg *__restrict__ segs, int nsegs,
+                  int units, int maxN, float h, const float *__restrict__ table) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  plane::Smem S;
+  float *exp, *rtab;
+  short *xmax;
+  plane::smem_layout<MODE>(S, dyn, maxN, exp, rtab, xmax);
+  plane::smem_init<MODE>(S, exp, table);
+  int have = -1;
+  for (int u = blockIdx.x; u < units; u += gridDim.x) {
+    int lo = 0, hi = nsegs - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (segs[mid].first <= u) lo = mid;
+      else hi = mid - 1;
+    }
+    const PlaneSeg g = segs[lo];
+    const InsertJob J = jobs[g.job];
+    if (have != g.job) {
+      __syncthreads();
+      plane::load_geometry(J, rtab, xmax);
+      __syncthreads();
+      have = g.job;
+    }
+    plane::slice_part<MODE>(J, S, (u - g.first) / g.parts, (u - g.first) % g.parts, g.parts, h,
+                            table);
+  }
+}
+
+// Adds a job's partial volume to its accumulators and clears it.  One block
+// per row; cells farther than the pixels and their windows reach are skipped.
+// The two self-conjugate cells keep a zero imaginary part once touched.
+__global__ void __launch_bounds__(128)
+    k_merge(float2 *__restrict__ data, float *__restrict__ norm, float2 *__restrict__ pdata,
+            float *__restrict__ pnorm, int N, float reach) {
+  const int w2 = N / 2 + 1;
+  const int y = blockIdx.x, z = blockIdx.y;
+  const float fy = (float)(y <= N / 2 ? y : y - N), fz = (float)(z <= N / 2 ? z : z - N);
+  const float left = reach * reach - fy * fy - fz * fz;
+  if (left < 0.0f) return;
+  const int n = min(w2, (int)sqrtf(left) + 2);
+  const size_t row = ((size_t)z * N + y) * w2;
+  for (int x = threadIdx.x; x < n; x += blockDim.x) {
+    const float s = pnorm[row + x];
+    const float2 v = pdata[row + x];
+    // (an x = 0 cell may hold conjugate values and no weight)
+    if (s == 0.0f && v.x == 0.0f && v.y == 0.0f) continue;
+    float2 d = data[row + x];
+    d.x += v.x;
+    d.y += v.y;
+    if (y == 0 && z == 0 && (x == 0 || x == w2 - 1)) d.y = 0.0f;
+    data[row + x] = d;
+    norm[row + x] += s;
+    pdata[row + x] = make_float2(0.0f, 0.0f);
+    pnorm[row + x] = 0.0f;
+  }
+}
+
+// Adds a job's centre copies to its accumulators and clears them: grid.y =
+// job, one thread per cell.
+__global__ void __launch_bounds__(256)
+    k_merge_centre(const InsertJob *__restrict__ jobs, const InsertJob one, int mode) {
+  const InsertJob &J = jobs ? jobs[blockIdx.y] : one;
+  if (!J.cdata || J.mode != mode) return;
+  const int c = J.centre, side = 2 * c + 1, N = J.N, w2 = N / 2 + 1;
+  const int cells = (c + 1) * side * side;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= cells) return;
+  float2 *cd = reinterpret_cast<float2 *>(J.cdata) + q;
+  float *cn = J.cdata + 2 * (size_t)J.copies * cells + q;
+  double re = 0.0, im = 0.0, w = 0.0;
+  bool any = false;
+  for (int k = 0; k < J.copies; k++, cd += cells, cn += cells) {
+    const float2 v = *cd;
+    const float s = *cn;
+    if (v.x == 0.0f && v.y == 0.0f && s == 0.0f) continue;
+    any = true;
+    re += v.x;
+    im += v.y;
+    w += s;
+    *cd = make_float2(0.0f, 0.0f);
+    *cn = 0.0f;
+  }
+  if (!any) return;
+  const int i = q % (c + 1), j = (q / (c + 1)) % side - c, l = q / ((c + 1) * side) - c;
+  const size_t at = (size_t)i + (size_t)((j < 0 ? N + j : j) + (l < 0 ? N + l : l) * N) * w2;
+  float2 *d = reinterpret_cast<float2 *>(J.fdata) + at;
+  float2 v = *d;
+  v.x += (float)re;
+  v.y = (i == 0 && j == 0 && l == 0) ? 0.0f : v.y + (float)im;
+  *d = v;
+  J.fnorm[at] += (float)w;
+}
+
+static int plane_parts(int N, int mode, long slices) {
+  // 8 x 4 patches of the bounding box of a slice's columns (at most, about
+  // N x N/2 * sqrt 2), eight to a block: a unit is small enough to balance
+  // the blocks and large enough to pay for its set-up
+  const int per = mode == MODE_GAUSS5 ? 8 : 32;
+  const long patches = (long)(N / 8 + 2) * (N / 4 + 3) * 3 / 4;
+  const long most = std::max(1L, (patches + plane::NW - 1) / plane::NW);
+  const long fine = std::max(1L, (patches + plane::NW * per - 1) / (plane::NW * per));
+  const long fill = (148L * 3 * 4 + slices - 1) / std::max(1L, slices);
+  return (int)std::min(most, std::max(fine, fill));
+}
+
+int plane_seg(const InsertJob &j, int job, int first, PlaneSeg &out) {
+  const long slices = (long)j.np * j.nsym;
+  out.job = job;
+  out.first = first;
+  out.parts = plane_parts(j.N, j.mode, slices);
+  const long end = first + slices * out.parts;
+  return end > INT_MAX ? -1 : (int)end;
+}
+
+// Blocks that fit the device at once, for a kernel and its shared memory
+// (looked up once: the query costs a small call a few microseconds).
+static int resident(const void *func, size_t smem, cudaError_t *e) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  static std::mutex mu;
+  static std::map<std::tuple<const void *, int, size_t>, int> known;
+  std::lock_guard<std::mutex> lk(mu);
+  int &n = known[std::make_tuple(func, dev, smem)];
+  *e = cudaSuccess;
+  if (n) return n;
+  *e = set_max_smem(func, smem);
+  if (*e != cudaSuccess) return 0;
+  int sms = 148, per_sm = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  *e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, plane::NT, smem);
+  if (*e != cudaSuccess) return 0;
+  return n = sms * std::max(1, per_sm);
+}
+
+template <int MODE>
+static cudaError_t launch_t(const InsertJob &j, float h, const float *table, cudaStream_t st) {
+  const long slices = (long)j.np * j.nsym;
+  const int parts = plane_parts(j.N, j.mode, slices);
+  if (slices * parts > INT_MAX) return cudaErrorInvalidValue;
+  const int units = (int)(slices * parts);
+  const size_t smem = plane::smem_bytes<MODE>(j.N);
+  cudaError_t e;
+  const int fit = resident((const void *)k_plane<MODE>, smem, &e);
+  if (e != cudaSuccess) return e;
+  note_launch();
+  k_plane<MODE><<<std::min(units, fit), plane::NT, smem, st>>>(j, units, parts, h, table);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_plane_tables(const InsertJob &j, const float *table, float h, cudaStream_t st) {
+  const long slices = (long)j.np * j.nsym;
+  if (slices == 0) return cudaSuccess;
+  if (plane_small(j.mode, j.N, slices)) return launch_scatter_tables(j, table, h, st);
+  switch (j.mode) {
+    case MODE_GAUSS2: return launch_t<MODE_GAUSS2>(j, h, table, st);
+    case MODE_GAUSS5: return launch_t<MODE_GAUSS5>(j, h, table, st);
+    case MODE_TRILINEAR: return launch_t<MODE_TRILINEAR>(j, h, table, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_plane(const InsertJob &j, cudaStream_t st) {
+  const Consts &c = consts();
+  return launch_plane_tables(j, c.d_exp, j.mode == MODE_GAUSS5 ? c.h5 : c.h2, st);
+}
+
+template <int MODE>
+static cudaError_t launch_multi_t(const InsertJob *d_jobs, const PlaneSeg *d_segs, int nsegs,
+                                  int units, int maxN, cudaStream_t st) {
+  const Consts &c = consts();
+  const size_t smem = plane::smem_bytes<MODE>(maxN);
+  cudaError_t e;
+  const int fit = resident((const void *)k_plane_multi<MODE>, smem, &e);
+  if (e != cudaSuccess) return e;
+  note_launch();
+  k_plane_multi<MODE><<<std::min(units, fit), plane::NT, smem, st>>>(
+      d_jobs, d_segs, nsegs, units, maxN, MODE == MODE_GAUSS5 ? c.h5 : c.h2, c.d_exp);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_plane_multi(const InsertJob *d_jobs, const PlaneSeg *d_segs, int nsegs,
+                               int units, int mode, int maxN, cudaStream_t st) {
+  if (units == 0) return cudaSuccess;
+  switch (mode) {
+    case MODE_GAUSS2: return launch_multi_t<MODE_GAUSS2>(d_jobs, d_segs, nsegs, units, maxN, st);
+    case MODE_GAUSS5: return launch_multi_t<MODE_GAUSS5>(d_jobs, d_segs, nsegs, units, maxN, st);
+    case MODE_TRILINEAR:
+      return launch_multi_t<MODE_TRILINEAR>(d_jobs, d_segs, nsegs, units, maxN, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+size_t plane_centre(int N, long slices, int &half, int &copies) {
+  half = std::min(15, N / 2 - 1);
+  copies = (int)std::min(32L, (std::min(slices, (long)kPlaneTurn) + 63) / 64);
+  return slices < 16 ? 0 : 12 * (size_t)copies * (half + 1) * (2 * half + 1) * (2 * half + 1);
+}
+
+cudaError_t launch_merge_centre(const InsertJob *d_jobs, int njobs, const InsertJob *one, int mode,
+                                int half, cudaStream_t st) {
+  const int cells = (half + 1) * (2 * half + 1) * (2 * half + 1);
+  note_launch();
+  k_merge_centre<<<dim3((cells + 255) / 256, njobs), 256, 0, st>>>(d_jobs, one ? *one : InsertJob(),
+                                                                   mode);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_merge(float *data, float *norm, float *pdata, float *pnorm, int N, int corners,
+                         cudaStream_t st) {
+  // the farthest pixel (the kernel takes matrices within 1 % of a rotation)
+  // and the corner of its window
+  const float reach = 1.01f * (corners ? 0.7072f * N + 1.0f : 0.5f * N + 0.52f) + 3.5f * 1.7321f;
+  note_launch();
+  k_merge<<<dim3(N, N), 128, 0, st>>>(reinterpret_cast<float2 *>(data), norm,
+                                      reinterpret_cast<float2 *>(pdata), pnorm, N, reach);
+  return cudaGetLastError();
+}
+
+}  // namespace fr

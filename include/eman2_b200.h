@@ -56,8 +56,8 @@ enum {
 /* Insertion schedules. */
 enum {
   FR_SCHED_AUTO = 0,     /* pick by batch size and mode */
-  FR_SCHED_SCATTER = 1,  /* one thread per slice pixel, FP32 atomics */
-  FR_SCHED_GATHER = 2    /* voxel tiles own their cells; no atomics */
+  FR_SCHED_SCATTER = 1,  /* slice by slice, FP32 atomics to the volume */
+  FR_SCHED_GATHER = 2    /* the tuned or default kernel for many slices */
 };
 
 /* FourierReconstructor parameters (libEM/reconstructor.h:501-516). */
@@ -344,8 +344,8 @@ FR_API int fr_batch_get_accumulators(fr_batch *b, int job, float *data, float *n
 /* Schedule selection for the insertion, measured on the device with
  * nparticles random slices and cached per (N, mode, nsym): candidates are the
  * register-tile gather shapes 0-3, the staged column kernel (4), the
- * barrier-free column kernel (5), the pixel-major kernel for windows one or
- * two taps wide (6; not for gauss_5) and the atomic scatter (tile_out = -2).
+ * mode's default kernel (5, and once more as 6; not for gauss_5) and the
+ * scatter schedule (tile_out = -2).
  * ms_out, if not NULL, receives 8 timings in that order (-1: not run).  fr_set_tile pins a
  * choice (-1 clears it).  No counterpart in the reference. */
 FR_API int fr_autotune(int N, int mode, int nsym, int nparticles, int *tile_out,
