@@ -1235,15 +1235,14 @@ int fr_determine_slice_agreement(fr_recon *r, const float *slices, int n, const 
   TRY(to_device(weights, sizeof(float) * n, r->s_w, st, &d_w));
   TRY(r->s_t3d.ensure(sizeof(float) * 9 * (size_t)n * r->nsym));
   CU(launch_compose((const float *)d_rot, r->d_sym.as<float>(), n, r->nsym, r->s_t3d.as<float>(), st));
+  // the blocks' sums, then the results when they go to the host
   const bool dev_out = is_device_ptr(out);
-  float *d_out = out;
-  if (!dev_out) {
-    TRY(r->s_out.ensure(sizeof(float) * 5 * n));
-    d_out = r->s_out.as<float>();
-  }
+  const size_t part = agree_scratch_bytes(N, n);
+  TRY(r->s_out.ensure(part + sizeof(float) * 5 * n));
+  float *d_out = dev_out ? out : reinterpret_cast<float *>(r->s_out.as<unsigned char>() + part);
   CU(launch_agree_rt(r->vol_data.as<float>(), r->vol_norm.as<float>(), N, (const float *)d_sl,
                      r->s_t3d.as<float>(), n, r->nsym, (const float *)d_w, apix, r->geom->d_rtab,
-                     d_out, st));
+                     r->s_out.as<double>(), d_out, st));
   if (!dev_out) TRY(from_device(out, d_out, sizeof(float) * 5 * n, st));
   else CU(cudaStreamSynchronize(st));
   return FR_OK;
