@@ -714,10 +714,16 @@ int prologue_run(PlanCache &plans, const ProScratch &b, const unsigned char *d_m
                  const PartSym *d_psym, long nslices) {
   const size_t img = (size_t)N * N, spec = (size_t)N * (N / 2 + 1);
   const MetaView mv = meta_view(d_meta, n);
-  TRY(b.img->ensure(sizeof(float) * img * n));
+  // sqrt(1.0f/ysize * xsize), applied before the r2c instead of after it
+  volatile float inv = 1.0f / (float)N;
+  const float scale = sqrtf(inv * (float)(N + 2));
   TRY(b.slices->ensure(sizeof(float) * slice_floats(N) * n));
-  TRY(b.spec->ensure(std::max(sizeof(cufftComplex) * spec, sizeof(float) * img) * n));
   TRY(b.t3d->ensure(sizeof(float) * 9 * (size_t)(nslices >= 0 ? nslices : (long)n * nsym)));
+  if (slice_fits(N, n, any_ctf))
+    return launch_slice(d_raw, d_src, n, box, N, any_ctf ? mv.ctf : nullptr, mv.txy, true, mv.rot,
+                        d_sym, nsym, b.t3d->as<float>(), d_psym, scale, b.slices->as<float2>(), st);
+  TRY(b.img->ensure(sizeof(float) * img * n));
+  TRY(b.spec->ensure(std::max(sizeof(cufftComplex) * spec, sizeof(float) * img) * n));
   if (any_ctf) TRY(b.img2->ensure(sizeof(float) * img * n));
   CU(launch_pad_compose(d_raw, d_src, n, box, N, b.img->as<float>(), mv.rot, d_sym, nsym,
                         b.t3d->as<float>(), st, d_psym));
@@ -731,8 +737,6 @@ int prologue_run(PlanCache &plans, const ProScratch &b, const unsigned char *d_m
   // edge mean (in the shift kernel); preprocess_slice: shift, phase origin
   // to corner, x sqrt((N+2)/N), r2c.  spec is the real staging for the r2c
   // input.
-  volatile float inv = 1.0f / (float)N;
-  const float scale = sqrtf(inv * (float)(N + 2));
   CU(launch_shift_corner(b.img->as<float>(), img_on, any_ctf ? mv.ctf : nullptr, nullptr, mv.txy,
                          2, n, N, scale, b.spec->as<float>(), st, true));
   TRY(plans.exec2d(true, N, n, b.spec->p, b.slices->p, st, exact_fft));
@@ -974,10 +978,13 @@ static int preprocess_device(fr_recon *r, const float *d_imgs, int n, const floa
                              int txy_stride, float *d_out_slices) {
   const int N = r->N;
   cudaStream_t st = r->stream;
-  TRY(r->s_img2.ensure(sizeof(float) * (size_t)n * N * N));
   // sqrt(1.0f/ysize * xsize) with ysize = N, xsize = N+2 (libEM/reconstructor.cpp:1054)
   volatile float inv = 1.0f / (float)N;
   const float scale = sqrtf(inv * (float)(N + 2));
+  if (slice_fits(N, n, false))
+    return launch_slice(d_imgs, nullptr, n, N, N, nullptr, d_txy, false, nullptr, nullptr, 0,
+                        nullptr, nullptr, scale, (float2 *)d_out_slices, st);
+  TRY(r->s_img2.ensure(sizeof(float) * (size_t)n * N * N));
   CU(launch_shift_corner(d_imgs, nullptr, nullptr, nullptr, d_txy, txy_stride, n, N, scale,
                          r->s_img2.as<float>(), st));
   TRY(r->plans.exec2d(true, N, n, r->s_img2.p, d_out_slices, st));

@@ -213,6 +213,14 @@ struct PartSym {
 cudaError_t launch_pad_compose(const float *d_raw, const float *const *d_src, int n, int box, int N,
                                float *d_img, const float *d_rot, const float *d_sym, int nsym,
                                float *d_t3d, cudaStream_t st, const PartSym *d_psym = nullptr);
+// The whole preparation of n particles in one launch (fr_slice.cu), where
+// slice_fits says that it is possible and the better way.  d_ctf, d_txy, d_rot null: no phase flip, no shift,
+// no composition; means: subtract the edge means.
+bool slice_fits(int N, int n, bool ctf);
+int launch_slice(const float *d_raw, const float *const *d_src, int n, int box, int N,
+                 const void *d_ctf, const float *d_txy, bool means, const float *d_rot,
+                 const float *d_sym, int nsym, float *d_t3d, const PartSym *d_psym,
+                 float scale_out, float2 *d_out, cudaStream_t st);
 void ctf_constants(float defocus, float dfdiff, float dfang, float voltage, float cs, float apix,
                    float ampcont, int N, void *out);
 size_t ctf_dev_size();

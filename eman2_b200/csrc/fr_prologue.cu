@@ -8,11 +8,13 @@
 //   recon.preprocess_slice(img, ts)         (libEM/reconstructor.cpp:1022-1061):
 //     bilinear xform (libEM/processor.cpp:11025-11080), phase origin to corner,
 //     r2c FFT, x sqrt((N+2)/N)
-// Here the FFTs are batched cuFFT plans and everything between them is one
-// kernel per stage over all particles of a chunk.
+// Here, for sizes fr_slice.cu does not take, the FFTs are batched cuFFT plans
+// and everything between them is one kernel per stage over all particles of a
+// chunk.
 #include <algorithm>
 #include <cmath>
 
+#include "fr_ctf.cuh"
 #include "fr_device.cuh"
 #include "fr_internal.h"
 
@@ -82,13 +84,7 @@ __global__ void __launch_bounds__(256) k_pad(const float *__restrict__ raw,
       s0 = (size_t)ps.slice0;
     }
     for (int t = threadIdx.x; t < ns * 9; t += blockDim.x) {
-      const int q = t / 9, e = t % 9, i = e / 3, j = e % 3;
-      const float *a = rot + 9 * (size_t)p;
-      const float *b = sy + 9 * q;
-      float v = __fmul_rn(a[3 * i + 0], b[j]);
-      v = __fadd_rn(v, __fmul_rn(a[3 * i + 1], b[3 + j]));
-      v = __fadd_rn(v, __fmul_rn(a[3 * i + 2], b[6 + j]));
-      t3d[(s0 + q) * 9 + e] = v;
+      t3d[s0 * 9 + t] = compose_element(rot + 9 * (size_t)p, sy + 9 * (t / 9), t % 9);
     }
   }
   const float *src = src_tab ? src_tab[p] : raw + (size_t)p * box * box;
@@ -126,19 +122,6 @@ cudaError_t launch_pad_compose(const float *d_raw, const float *const *d_src, in
   return cudaGetLastError();
 }
 
-// Util::hypot_fast value: std::hypot(float,float) of small integers, which
-// glibc evaluates as a double square root rounded once to float.
-__device__ __forceinline__ float hypot_int(int x, int y) {
-  return (float)sqrt((double)(x * x + y * y));
-}
-
-// x CTF_SIGN(defocus) on r2c spectra (n, N, N/2+1).  The per-particle
-// constants (g1, g2, acac, ds) are formed on the host exactly as
-// EMAN2Ctf::compute_2d_complex forms them; the sign of cos(gam - acac) is
-// taken from a double cosine of the float argument, which is the sign the
-// correctly rounded float cosine returns.
-struct CtfDev { float g1, g2, acac, ds, defocus, dfdiff, dfang, on; };
-
 // Blocks of 256 threads per particle for a launch over n particles of npx
 // elements each: about `waves` blocks per SM in all, at most one element
 // per thread.  Few particles get many blocks each; many get one.
@@ -154,20 +137,7 @@ static int blocks_per_particle(int n, int npx, int waves) {
 // frequency.
 __device__ __forceinline__ void flip_one(cufftComplex *__restrict__ spec, const CtfDev &k, int N,
                                          int i, int r, int x) {
-  const int y = r < N / 2 ? r : r - N;
-  const float s = __fmul_rn(hypot_int(x, y), k.ds);
-  float gam;
-  const float t1 = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(-k.g1, s), s), s), s);
-  if (k.dfdiff == 0.0f) {
-    gam = __fadd_rn(t1, __fmul_rn(__fmul_rn(__fmul_rn(k.g2, k.defocus), s), s));
-  } else {
-    const float ang = atan2f((float)y, (float)x);
-    const double a2 = (double)__fmul_rn(2.0f, ang) - 2.0 * 3.14159265358979323846 / 180.0f * (double)k.dfang;
-    const float df = (float)((double)k.defocus + (double)(k.dfdiff / 2.0f) * cos(a2));
-    gam = __fadd_rn(t1, __fmul_rn(__fmul_rn(__fmul_rn(k.g2, df), s), s));
-  }
-  const double v = cos((double)__fsub_rn(gam, k.acac));
-  const float sg = v < 0.0 ? -1.0f : 1.0f;
+  const float sg = ctf_sign(k, x, r < N / 2 ? r : r - N);
   cufftComplex z = spec[i];
   z.x = __fmul_rn(z.x, sg);
   z.y = __fmul_rn(z.y, sg);

@@ -1,0 +1,69 @@
+"""The one-launch particle preparation (fr_slice.cu) over radix pairs of every
+kind (equal, unequal, odd with even, the largest image that fits), odd and
+oversized boxes, shifts from none to beyond the image, and particles with and
+without a phase flip in one call.  FP32 transforms against FP64 ones rounded:
+2e-5 as for the other FFT paths (a transform's error is a few eps log2 N)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+RTOL = 2e-5
+
+
+def _shifts(n, N, rng):
+    s = rng.uniform(-5, 5, (n, 2)).astype(np.float32)
+    fixed = [(0, 0), (0, 1.5), (-2.25, 0), (3, -4), (1e-7, -1e-7), (-0.5, 2e-6), (N / 2, 0.25),
+             (0.75, -N), (-1.0 * N, 2.0), (-0.999999, 0.999999)]
+    s[:len(fixed)] = np.asarray(fixed, np.float32)
+    return s
+
+
+@pytest.mark.parametrize("N", [16, 18, 30, 42, 84, 98, 150, 196, 240])
+def test_preprocess_sizes(gpu, N):
+    from eman2_b200 import Reconstructors, _lib
+    n = 48
+    rng = np.random.default_rng(N)
+    img = rng.normal(size=(n, N, N)).astype(np.float32)
+    inv = _shifts(n, N, rng)
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
+    r.setup()
+    out = np.empty((n, N, N + 2), np.float32)
+    _lib.check(_lib.load().fr_preprocess_slices(r.handle, _lib.ptr(img), n, _lib.ptr(inv),
+                                                _lib.ptr(out)))
+    for i in range(n):
+        want = oracle.preprocess_slice(img[i], float(inv[i, 0]), float(inv[i, 1]))
+        if not want.any():
+            assert not out[i].any()
+        else:
+            assert oracle.rel_l2(out[i], want) < RTOL, i
+
+
+@pytest.mark.parametrize("box,N", [(11, 16), (64, 96), (101, 150), (33, 32), (70, 60), (128, 192),
+                                   (160, 240)])
+def test_particles_sizes(gpu, box, N):
+    from eman2_b200 import Reconstructors
+    from eman2_b200.particles import particle_meta
+    from eman2_b200.synth import quaternion_blocks, random_quaternions
+    n = 48
+    rng = np.random.default_rng(N + 1)
+    img = (rng.normal(size=(n, box, box)) + 3.0).astype(np.float32)
+    rots = quaternion_blocks(random_quaternions(n, rng))
+    shifts = rng.uniform(-3, 3, (n, 2)).astype(np.float32)
+    w = rng.uniform(0.5, 1.0, n).astype(np.float32)
+    df = rng.uniform(0.8, 2.5, n).astype(np.float32)
+    df[::5] = 0.0
+    ctf = {"dfdiff": 0.1, "dfang": 30.0}
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
+    r.setup()
+    r.insert_particles(img, particle_meta(rots, shifts, w, ctf=ctf, defocus=df))
+    d, nm = r.get_accumulators()
+    sl = np.stack([oracle.particle_to_slice(img[i], N, shifts[i], dict(ctf, defocus=float(df[i])))
+                   for i in range(n)])
+    o = oracle.OracleVolume(N, "fp32acc64")
+    o.insert(sl, rots, w, "gauss_2", "c1")
+    assert oracle.rel_l2(nm, o.norm) < 2e-6
+    assert oracle.rel_l2(d, o.data) < RTOL
