@@ -315,6 +315,21 @@ bool is_device_ptr(const void *p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Page-locked host memory (cudaHostAlloc / cudaHostRegister): the copy
+// engine reads and writes it without a staging copy, so copies into it are
+// asynchronous.
+static bool is_pinned_host(const void *p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
+// Host inputs up to this size go through a pinned ring in one upload.
+constexpr size_t kSmallUpload = 1u << 20;
+
 // Device view of a caller buffer: device pointers pass through; host buffers
 // are copied into `stage` on `st`.
 int to_device(const void *src, size_t bytes, DevBuf &stage, cudaStream_t st,
@@ -331,6 +346,7 @@ int from_device(void *dst, const void *dsrc, size_t bytes, cudaStream_t st) {
     CU(cudaMemcpyAsync(dst, dsrc, bytes, cudaMemcpyDeviceToDevice, st));
     CU(cudaStreamSynchronize(st));
   } else {
+    if (!is_pinned_host(dst) && copy_to_pageable(dst, dsrc, bytes, st)) return FR_OK;
     CU(cudaMemcpyAsync(dst, dsrc, bytes, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
   }
@@ -677,8 +693,13 @@ bool prologue_meta_range(int N, int n, int first, int count, const fr_particle *
   bool any_ctf = false;
   for (int i = first; i < first + count; i++) {
     const fr_particle &m = meta[i - first];
-    ctf_constants(m.defocus, m.dfdiff, m.dfang, m.voltage, m.cs, m.apix, m.ampcont, N,
-                  blk + cs * i);
+    // a stack's particles share their microscope: its constants once
+    const fr_particle *q = i > first ? &meta[i - first - 1] : nullptr;
+    if (q && q->voltage == m.voltage && q->cs == m.cs && q->apix == m.apix && q->ampcont == m.ampcont)
+      ctf_constants_as(m.defocus, m.dfdiff, m.dfang, blk + cs * (i - 1), blk + cs * i);
+    else
+      ctf_constants(m.defocus, m.dfdiff, m.dfang, m.voltage, m.cs, m.apix, m.ampcont, N,
+                    blk + cs * i);
     if (std::fabs(m.defocus) > 1e-4f) any_ctf = true;
     // ts = inverse of the translation-only part of xform.projection; the
     // bilinear xform then applies ts^-1, i.e. +(tx, ty) (programs/e2spa_make3d.py:339-342).
@@ -857,6 +878,7 @@ int fr_create(const fr_params *p, fr_recon **out) {
     delete r;
     return fail(FR_ECUDA, "cudaEventCreate failed: %s", cudaGetErrorString(cudaGetLastError()));
   }
+  host_pool_enter();
   consts();
   r->geom = get_geom(r->N, p->mode == FR_MODE_ITER ? 3 : p->corners);
   *out = r;
@@ -890,6 +912,7 @@ int fr_destroy(fr_recon *r) {
     r->done.reset();
     if (r->own) cudaStreamDestroy(r->own);
   }
+  host_pool_leave();
   delete r;
   return FR_OK;
 }
@@ -1001,8 +1024,24 @@ int fr_preprocess_slices(fr_recon *r, const float *imgs, int n, const float *inv
   TRY(stream_enter(r, r->stream));
   const int N = r->N;
   const void *d_in = nullptr, *d_t = nullptr;
-  TRY(to_device(imgs, sizeof(float) * (size_t)n * N * N, r->s_in, r->stream, &d_in));
-  if (inv_txy) TRY(to_device(inv_txy, sizeof(float) * 2 * n, r->s_txy, r->stream, &d_t));
+  const size_t ibytes = sizeof(float) * (size_t)n * N * N, tbytes = sizeof(float) * 2 * (size_t)n;
+  if (ibytes <= kSmallUpload && !is_device_ptr(imgs) && !(inv_txy && is_device_ptr(inv_txy))) {
+    // an image or a few from the host: one upload through the pinned ring
+    int slot;
+    unsigned char *blk;
+    const size_t all = ibytes + (inv_txy ? tbytes : 0);
+    TRY(r->s_in.ensure(all));
+    TRY(r->ring_small.acquire(all, &slot, &blk));
+    memcpy(blk, imgs, ibytes);
+    if (inv_txy) memcpy(blk + ibytes, inv_txy, tbytes);
+    CU(cudaMemcpyAsync(r->s_in.p, blk, all, cudaMemcpyHostToDevice, r->stream));
+    TRY(r->ring_small.done(slot, r->stream));
+    d_in = r->s_in.p;
+    if (inv_txy) d_t = r->s_in.as<unsigned char>() + ibytes;
+  } else {
+    TRY(to_device(imgs, ibytes, r->s_in, r->stream, &d_in));
+    if (inv_txy) TRY(to_device(inv_txy, tbytes, r->s_txy, r->stream, &d_t));
+  }
   const bool dev_out = is_device_ptr(out_slices);
   float *d_out = out_slices;
   if (!dev_out) {
@@ -1049,8 +1088,30 @@ int fr_insert_slices(fr_recon *r, const float *slices, int n, const float *rot, 
     if (status_out) status_out[i] = (w[i] == 0.0f) ? -1 : 0;
   const bool use_ssnr = any_neg;
   const void *d_sl = nullptr, *d_rot = nullptr, *d_ss = nullptr;
-  TRY(to_device(slices, sizeof(float) * slice_floats(N) * n, r->s_in, st, &d_sl));
-  TRY(to_device(rot, sizeof(float) * 9 * n, r->s_rot, st, &d_rot));
+  const size_t sbytes = sizeof(float) * slice_floats(N) * n, rbytes = sizeof(float) * 9 * (size_t)n;
+  if (!use_ssnr && sbytes <= kSmallUpload && !is_device_ptr(slices) && !is_device_ptr(rot)) {
+    // a slice or a few from the host: one upload through the pinned ring, and
+    // nothing left to wait for (insert_slice's loop goes on to its next image)
+    int slot;
+    unsigned char *blk;
+    const size_t wbytes = sizeof(float) * (size_t)n, all = sbytes + rbytes + wbytes;
+    TRY(r->s_in.ensure(all));
+    TRY(r->ring_small.acquire(all, &slot, &blk));
+    memcpy(blk, slices, sbytes);
+    memcpy(blk + sbytes, rot, rbytes);
+    memcpy(blk + sbytes + rbytes, w.data(), wbytes);
+    CU(cudaMemcpyAsync(r->s_in.p, blk, all, cudaMemcpyHostToDevice, st));
+    TRY(r->ring_small.done(slot, st));
+    const unsigned char *d = r->s_in.as<unsigned char>();
+    TRY(r->s_t3d.ensure(sizeof(float) * 9 * (size_t)n * r->nsym));
+    CU(launch_compose((const float *)(d + sbytes), r->d_sym.as<float>(), n, r->nsym,
+                      r->s_t3d.as<float>(), st));
+    TRY(insert_device(r, (const float2 *)d, r->s_t3d.as<float>(),
+                      (const float *)(d + sbytes + rbytes), n, schedule, nullptr, 0));
+    return stream_leave(r, st);
+  }
+  TRY(to_device(slices, sbytes, r->s_in, st, &d_sl));
+  TRY(to_device(rot, rbytes, r->s_rot, st, &d_rot));
   if (use_ssnr)
     TRY(to_device(ssnr, sizeof(float) * (size_t)nssnr * n, r->s_ssnr, st, &d_ss));
   TRY(r->s_w.ensure(sizeof(float) * n));
@@ -1344,18 +1405,6 @@ int fr_finish(fr_recon *r, int doift, float *out, float *normout) {
   CU(cudaStreamSynchronize(st));
   r->state = 2;
   return FR_OK;
-}
-
-// Page-locked host memory (cudaHostAlloc / cudaHostRegister): the copy
-// engine reads and writes it without a staging copy, so copies into it are
-// asynchronous.
-static bool is_pinned_host(const void *p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return a.type == cudaMemoryTypeHost;
 }
 
 int fr_finish_async(fr_recon *r, int doift, float *out, float *normout, void *stream) {

@@ -164,6 +164,10 @@ struct SharedEvent {
 bool is_device_ptr(const void *p);
 int to_device(const void *src, size_t bytes, DevBuf &stage, cudaStream_t st, const void **out);
 int from_device(void *dst, const void *dsrc, size_t bytes, cudaStream_t st);
+// fr_host.cu: large results to pageable memory; the pool's users are the handles.
+bool copy_to_pageable(void *dst, const void *dsrc, size_t bytes, cudaStream_t st);
+void host_pool_enter();
+void host_pool_leave();
 
 // ------------------------------------------------------------- cuFFT plans
 // Plans made with cuFFT's own work-area allocation turned off: every plan of

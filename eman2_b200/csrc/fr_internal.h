@@ -223,6 +223,8 @@ int launch_slice(const float *d_raw, const float *const *d_src, int n, int box, 
                  float scale_out, float2 *d_out, cudaStream_t st);
 void ctf_constants(float defocus, float dfdiff, float dfang, float voltage, float cs, float apix,
                    float ampcont, int N, void *out);
+// The same for a particle whose other constants are those at `from`.
+void ctf_constants_as(float defocus, float dfdiff, float dfang, const void *from, void *out);
 size_t ctf_dev_size();
 cudaError_t launch_ctf_flip_dev(cufftComplex *d_spec, const void *d_ctf, int n, int N,
                                 cudaStream_t st);

@@ -193,6 +193,14 @@ void ctf_constants(float defocus, float dfdiff, float dfang, float voltage, floa
   k.dfang = dfang;
   k.on = fabsf(defocus) > 1e-4f ? 1.0f : 0.0f;
 }
+void ctf_constants_as(float defocus, float dfdiff, float dfang, const void *from, void *out) {
+  CtfDev k = *reinterpret_cast<const CtfDev *>(from);
+  k.defocus = defocus;
+  k.dfdiff = dfdiff;
+  k.dfang = dfang;
+  k.on = fabsf(defocus) > 1e-4f ? 1.0f : 0.0f;
+  *reinterpret_cast<CtfDev *>(out) = k;
+}
 size_t ctf_dev_size() { return sizeof(CtfDev); }
 
 // Per-particle image source after the optional CTF round trip: particles

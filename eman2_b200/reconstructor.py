@@ -449,6 +449,18 @@ class FourierReconstructor:
         _lib.check(_lib.load().fr_get_accumulators(self._h, _lib.ptr(d), _lib.ptr(n)))
         return d, n
 
+    def _norm_array(self):
+        """Where the weight volume goes, if "normout" or "savenorm" asks for it."""
+        if isinstance(self.params.get("normout"), EMData) or self.params.get("savenorm"):
+            return np.empty((self.NZ, self.N, self.N // 2 + 1), np.float32)
+        return None
+
+    def _keep_norm(self, norm):
+        if isinstance(self.params.get("normout"), EMData):
+            self.params["normout"].set_data(norm)
+        if self.params.get("savenorm"):
+            np.save(str(self.params["savenorm"]), norm)
+
     def finish(self, doift: bool = True) -> EMData:
         """FourierReconstructor::finish (libEM/reconstructor.cpp:1552-1641).
         doift: real N^3 map (phase origin at the centre); else the normalised
@@ -457,13 +469,10 @@ class FourierReconstructor:
             self._require_setup()
         N, NZ = self.N, self.NZ
         out = np.empty((NZ, N, N) if doift else (NZ, N, N + 2), np.float32)
-        norm = np.empty((NZ, N, N // 2 + 1), np.float32)
+        norm = self._norm_array()
         _lib.check(_lib.load().fr_finish(self._h, int(bool(doift)), _lib.ptr(out), _lib.ptr(norm)))
         self._state = 2
-        if "normout" in self.params and isinstance(self.params["normout"], EMData):
-            self.params["normout"].set_data(norm)
-        if self.params.get("savenorm"):
-            np.save(str(self.params["savenorm"]), norm)
+        self._keep_norm(norm)
         return EMData(out, is_complex=not doift)
 
     def finish_async(self, doift: bool = True, stream=None) -> "PendingFinish":
@@ -510,14 +519,11 @@ class FourierReconstructor:
             outsize = (int(outsize),) * 3
         ox, oy, oz = (int(v) for v in outsize)
         out = np.empty((oz, oy, ox), np.float32)
-        norm = np.empty((N, N, N // 2 + 1), np.float32)
+        norm = self._norm_array()
         _lib.check(_lib.load().fr_finish_corrected(self._h, float(gauss_width), ox, oy, oz,
                                                    _lib.ptr(out), _lib.ptr(norm)))
         self._state = 2
-        if "normout" in self.params and isinstance(self.params["normout"], EMData):
-            self.params["normout"].set_data(norm)
-        if self.params.get("savenorm"):
-            np.save(str(self.params["savenorm"]), norm)
+        self._keep_norm(norm)
         return EMData(out)
 
     def _require_setup(self):

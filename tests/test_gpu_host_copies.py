@@ -1,0 +1,59 @@
+"""Results into pageable host memory: byte for byte what the device holds, for
+sizes around the pieces the copying threads take and from several host threads
+at once; and finish() with and without the weight volume asked for."""
+from __future__ import annotations
+
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _seeded(N, seed):
+    from eman2_b200 import Reconstructors
+    rng = np.random.default_rng(seed)
+    d = rng.normal(size=(N, N, N + 2)).astype(np.float32)
+    w = rng.uniform(0.5, 2.0, (N, N, N // 2 + 1)).astype(np.float32)
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
+    r.setup_seedandweights(d, w)
+    return r, d, w
+
+
+@pytest.mark.parametrize("N", [16, 100, 102, 126, 128, 160, 254])
+def test_accumulators_round_trip(gpu, N):
+    r, d, w = _seeded(N, N)
+    gd, gw = r.get_accumulators()
+    assert np.array_equal(gd, d) and np.array_equal(gw, w)
+
+
+def test_round_trips_from_threads(gpu):
+    jobs = [_seeded(N, N) for N in (128, 140, 160, 130)]
+    bad = []
+
+    def run(r, d, w):
+        for _ in range(5):
+            gd, gw = r.get_accumulators()
+            if not (np.array_equal(gd, d) and np.array_equal(gw, w)):
+                bad.append(d.shape)
+
+    ts = [threading.Thread(target=run, args=j) for j in jobs]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+
+
+def test_finish_weights_only_when_asked(gpu, tmp_path):
+    from eman2_b200 import EMData
+    r, _, _ = _seeded(48, 1)
+    plain = r.finish(True).numpy()
+    out = EMData(nx=1, ny=1)
+    for key, val in (("normout", out), ("savenorm", str(tmp_path / "n.npy"))):
+        r, _, _ = _seeded(48, 1)
+        r.insert_params({key: val})
+        assert np.array_equal(r.finish(True).numpy(), plain)
+    assert np.array_equal(out.numpy(), np.load(tmp_path / "n.npy"))
+    assert out.numpy().shape == (48, 48, 25)
