@@ -20,12 +20,13 @@
 // six taps, the weights go through packed operations, and a cell leaves the
 // registers once.
 // Measured on one B200, insertion alone (the kernels it took over from in
-// parentheses): gauss_5, d7, N = 384, 64 particles 21.3 ms (46.8, tile columns
+// parentheses): gauss_5, d7, N = 384, 64 particles 20.1 ms (46.8, tile columns
 // with shared read-modify-writes), one particle 0.43 ms (1.32, an atomic per
-// tap); gauss_2, c1, N = 192, 2048 particles 1.42 ms (2.12, tiles with shared
-// atomics).  Shared memory: three blocks of eight warps fit an SM at gauss_5's
-// 72 KB and 80 registers; more blocks at fewer registers spilled (gauss_2 at 4
-// and 5 blocks: 1.60 and 1.71 ms).
+// tap); gauss_2, c1, N = 192, 2048 particles 1.52 ms (2.12, tiles with shared
+// atomics).  Blocks an SM: gauss_5 without spills (two of eight warps, 128
+// registers) against three at 80, 20.1 against 21.6 ms; five or four of four
+// warps 20.8 and 20.3.  The two-tap windows at three blocks 1.52 ms, two 1.70,
+// four 1.60, five 1.71 (spills).
 //
 // Tap selection and weights are the reference's bit for bit (window start,
 // exp-table index, radius); a cell's taps of one slice are summed before they
@@ -48,8 +49,6 @@
 namespace fr {
 namespace plane {
 
-constexpr int NT = 256;         // threads: 8 independent warps
-constexpr int NW = NT / 32;
 constexpr float kDel = 0.02f;   // slack on the approximate plane geometry
 
 // Taps of a window along one axis, its reach (a pixel at p covers tap t iff
@@ -62,11 +61,11 @@ constexpr float kDel = 0.02f;   // slack on the approximate plane geometry
 template <int MODE> struct Win;
 template <> struct Win<MODE_GAUSS5> {
   static constexpr float lo = 2.5f, hi = 3.5f;
-  static constexpr int K = 6, W = 20, CTAS = 3, EXP = 2048;
+  static constexpr int K = 6, W = 20, EXP = 2048, NT = 256, CTAS = 2;
 };
 template <> struct Win<MODE_GAUSS2> {
   static constexpr float lo = 1.0f, hi = 1.0f;
-  static constexpr int K = 2, W = 8, CTAS = 3, EXP = 512;
+  static constexpr int K = 2, W = 8, EXP = 512, NT = 256, CTAS = 3;
 };
 template <> struct Win<MODE_TRILINEAR> : Win<MODE_GAUSS2> {
   static constexpr int EXP = 0;
@@ -408,6 +407,7 @@ template <int MODE>
 __device__ __forceinline__ void slice_part(const InsertJob &J, const Smem &S, int s, int part,
                                            int parts, float h, const float *__restrict__ table) {
   constexpr float LO = Win<MODE>::lo, HI = Win<MODE>::hi;
+  constexpr int NT = Win<MODE>::NT, NW = NT / 32;
   const int N = J.N, n2 = N >> 1, w2 = n2 + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int p = s / J.nsym;
@@ -508,7 +508,7 @@ __device__ __forceinline__ void slice_part(const InsertJob &J, const Smem &S, in
 template <int MODE>
 __device__ __forceinline__ void smem_layout(Smem &S, unsigned char *dyn, int maxN, float *&exp,
                                             float *&rtab, short *&xmax) {
-  constexpr int W = Win<MODE>::W;
+  constexpr int W = Win<MODE>::W, NW = Win<MODE>::NT / 32;
   const int warp = threadIdx.x >> 5;
   S.geom = reinterpret_cast<SliceGeom *>(dyn) + warp;
   float2 *sv = reinterpret_cast<float2 *>(dyn + NW * sizeof(SliceGeom));
@@ -524,6 +524,7 @@ __device__ __forceinline__ void smem_layout(Smem &S, unsigned char *dyn, int max
 }
 
 template <int MODE> size_t smem_bytes(int maxN) {
+  constexpr int NW = Win<MODE>::NT / 32;
   return NW * sizeof(SliceGeom) + (size_t)NW * Win<MODE>::W * 32 * 12 + Win<MODE>::EXP * 4 +
          4 * (size_t)(maxN + 2) + 2 * (size_t)maxN;
 }
@@ -531,7 +532,7 @@ template <int MODE> size_t smem_bytes(int maxN) {
 template <int MODE>
 __device__ __forceinline__ void smem_init(const Smem &S, float *exp,
                                           const float *__restrict__ table) {
-  for (int i = threadIdx.x; i < Win<MODE>::EXP; i += NT) exp[i] = i < 1000 ? __ldg(&table[i]) : 0.0f;
+  for (int i = threadIdx.x; i < Win<MODE>::EXP; i += Win<MODE>::NT) exp[i] = i < 1000 ? __ldg(&table[i]) : 0.0f;
   for (int i = threadIdx.x & 31; i < Win<MODE>::W * 32; i += 32) {
     S.sv[i] = make_float2(0.0f, 0.0f);
     S.sw[i] = 0.0f;
@@ -539,15 +540,15 @@ __device__ __forceinline__ void smem_init(const Smem &S, float *exp,
 }
 
 __device__ __forceinline__ void load_geometry(const InsertJob &J, float *rtab, short *xmax) {
-  for (int i = threadIdx.x; i < J.N + 2; i += NT) rtab[i] = __ldg(&J.rtab[i]);
-  for (int i = threadIdx.x; i < J.N; i += NT) xmax[i] = (short)__ldg(&J.xmax[i]);
+  for (int i = threadIdx.x; i < J.N + 2; i += blockDim.x) rtab[i] = __ldg(&J.rtab[i]);
+  for (int i = threadIdx.x; i < J.N; i += blockDim.x) xmax[i] = (short)__ldg(&J.xmax[i]);
 }
 
 }  // namespace plane
 
 // One job: unit u is part u % parts of slice u / parts.
 template <int MODE>
-__global__ void __launch_bounds__(plane::NT, plane::Win<MODE>::CTAS)
+__global__ void __launch_bounds__(plane::Win<MODE>::NT, plane::Win<MODE>::CTAS)
     k_plane(InsertJob J, int units, int parts, float h, const float *__restrict__ table) {
   extern __shared__ __align__(16) unsigned char dyn[];
   plane::Smem S;
@@ -563,7 +564,7 @@ __global__ void __launch_bounds__(plane::NT, plane::Win<MODE>::CTAS)
 
 // Several jobs of one mode: job segs[i].job has the units from segs[i].first on.
 template <int MODE>
-__global__ void __launch_bounds__(plane::NT, plane::Win<MODE>::CTAS)
+__global__ void __launch_bounds__(plane::Win<MODE>::NT, plane::Win<MODE>::CTAS)
     k_plane_multi(const InsertJob *__restrict__ jobs, const PlaneSeg *__restrict__ segs, int nsegs,
                   int units, int maxN, float h, const float *__restrict__ table) {
   extern __shared__ __align__(16) unsigned char dyn[];
@@ -660,13 +661,13 @@ __global__ void __launch_bounds__(256)
 
 static int plane_parts(int N, int mode, long slices) {
   // 8 x 4 patches of the bounding box of a slice's columns (at most, about
-  // N x N/2 * sqrt 2), eight to a block: a unit is small enough to balance
-  // the blocks and large enough to pay for its set-up
-  const int per = mode == MODE_GAUSS5 ? 8 : 32;
+  // N x N/2 * sqrt 2), one to a warp at a time: a unit (a block's share) is
+  // small enough to balance the blocks and large enough to pay for its set-up
+  const int warps = 8, per = mode == MODE_GAUSS5 ? 8 : 32;
   const long patches = (long)(N / 8 + 2) * (N / 4 + 3) * 3 / 4;
-  const long most = std::max(1L, (patches + plane::NW - 1) / plane::NW);
-  const long fine = std::max(1L, (patches + plane::NW * per - 1) / (plane::NW * per));
-  const long fill = (148L * 3 * 4 + slices - 1) / std::max(1L, slices);
+  const long most = std::max(1L, (patches + warps - 1) / warps);
+  const long fine = std::max(1L, (patches + warps * per - 1) / (warps * per));
+  const long fill = (148L * 12 + slices - 1) / std::max(1L, slices);
   return (int)std::min(most, std::max(fine, fill));
 }
 
@@ -681,7 +682,7 @@ int plane_seg(const InsertJob &j, int job, int first, PlaneSeg &out) {
 
 // Blocks that fit the device at once, for a kernel and its shared memory
 // (looked up once: the query costs a small call a few microseconds).
-static int resident(const void *func, size_t smem, cudaError_t *e) {
+static int resident(const void *func, int threads, size_t smem, cudaError_t *e) {
   int dev = 0;
   cudaGetDevice(&dev);
   static std::mutex mu;
@@ -694,7 +695,7 @@ static int resident(const void *func, size_t smem, cudaError_t *e) {
   if (*e != cudaSuccess) return 0;
   int sms = 148, per_sm = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  *e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, plane::NT, smem);
+  *e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, threads, smem);
   if (*e != cudaSuccess) return 0;
   return n = sms * std::max(1, per_sm);
 }
@@ -707,10 +708,10 @@ static cudaError_t launch_t(const InsertJob &j, float h, const float *table, cud
   const int units = (int)(slices * parts);
   const size_t smem = plane::smem_bytes<MODE>(j.N);
   cudaError_t e;
-  const int fit = resident((const void *)k_plane<MODE>, smem, &e);
+  const int fit = resident((const void *)k_plane<MODE>, plane::Win<MODE>::NT, smem, &e);
   if (e != cudaSuccess) return e;
   note_launch();
-  k_plane<MODE><<<std::min(units, fit), plane::NT, smem, st>>>(j, units, parts, h, table);
+  k_plane<MODE><<<std::min(units, fit), plane::Win<MODE>::NT, smem, st>>>(j, units, parts, h, table);
   return cudaGetLastError();
 }
 
@@ -737,10 +738,10 @@ static cudaError_t launch_multi_t(const InsertJob *d_jobs, const PlaneSeg *d_seg
   const Consts &c = consts();
   const size_t smem = plane::smem_bytes<MODE>(maxN);
   cudaError_t e;
-  const int fit = resident((const void *)k_plane_multi<MODE>, smem, &e);
+  const int fit = resident((const void *)k_plane_multi<MODE>, plane::Win<MODE>::NT, smem, &e);
   if (e != cudaSuccess) return e;
   note_launch();
-  k_plane_multi<MODE><<<std::min(units, fit), plane::NT, smem, st>>>(
+  k_plane_multi<MODE><<<std::min(units, fit), plane::Win<MODE>::NT, smem, st>>>(
       d_jobs, d_segs, nsegs, units, maxN, MODE == MODE_GAUSS5 ? c.h5 : c.h2, c.d_exp);
   return cudaGetLastError();
 }
