@@ -743,6 +743,16 @@ int prologue_run(PlanCache &plans, const ProScratch &b, const unsigned char *d_m
   if (slice_fits(N, n, any_ctf))
     return launch_slice(d_raw, d_src, n, box, N, any_ctf ? mv.ctf : nullptr, mv.txy, true, mv.rot,
                         d_sym, nsym, b.t3d->as<float>(), d_psym, scale, b.slices->as<float2>(), st);
+  if (lines_fits(N, n)) {
+    if (any_ctf) {
+      TRY(b.img->ensure(sizeof(float) * img * n));
+      TRY(b.spec->ensure(lines_edge_bytes(N, n)));
+    }
+    return launch_lines(d_raw, d_src, n, box, N, any_ctf ? mv.ctf : nullptr, mv.txy, true, mv.rot,
+                        d_sym, nsym, b.t3d->as<float>(), d_psym, scale,
+                        any_ctf ? b.img->as<float>() : nullptr,
+                        any_ctf ? b.spec->as<double>() : nullptr, b.slices->as<float2>(), st);
+  }
   TRY(b.img->ensure(sizeof(float) * img * n));
   TRY(b.spec->ensure(std::max(sizeof(cufftComplex) * spec, sizeof(float) * img) * n));
   if (any_ctf) TRY(b.img2->ensure(sizeof(float) * img * n));
@@ -1004,9 +1014,19 @@ static int preprocess_device(fr_recon *r, const float *d_imgs, int n, const floa
   // sqrt(1.0f/ysize * xsize) with ysize = N, xsize = N+2 (libEM/reconstructor.cpp:1054)
   volatile float inv = 1.0f / (float)N;
   const float scale = sqrtf(inv * (float)(N + 2));
-  if (slice_fits(N, n, false))
+  // These two write slices while images are still to be read, as pairs of
+  // floats; images and slices that share memory, or slices at an odd float,
+  // take the staged path.
+  const char *in = (const char *)d_imgs, *out = (const char *)d_out_slices;
+  const bool direct = (uintptr_t)out % sizeof(float2) == 0 &&
+                      (out >= in + sizeof(float) * (size_t)n * N * N ||
+                       in >= out + sizeof(float) * slice_floats(N) * n);
+  if (direct && slice_fits(N, n, false))
     return launch_slice(d_imgs, nullptr, n, N, N, nullptr, d_txy, false, nullptr, nullptr, 0,
                         nullptr, nullptr, scale, (float2 *)d_out_slices, st);
+  if (direct && lines_fits(N, n))
+    return launch_lines(d_imgs, nullptr, n, N, N, nullptr, d_txy, false, nullptr, nullptr, 0,
+                        nullptr, nullptr, scale, nullptr, nullptr, (float2 *)d_out_slices, st);
   TRY(r->s_img2.ensure(sizeof(float) * (size_t)n * N * N));
   CU(launch_shift_corner(d_imgs, nullptr, nullptr, nullptr, d_txy, txy_stride, n, N, scale,
                          r->s_img2.as<float>(), st));

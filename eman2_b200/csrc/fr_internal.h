@@ -221,6 +221,14 @@ int launch_slice(const float *d_raw, const float *const *d_src, int n, int box, 
                  const void *d_ctf, const float *d_txy, bool means, const float *d_rot,
                  const float *d_sym, int nsym, float *d_t3d, const PartSym *d_psym,
                  float scale_out, float2 *d_out, cudaStream_t st);
+// The same in up to five launches (fr_lines.cu), where lines_fits says so;
+// d_img, d_edge: n images and lines_edge_bytes of workspace, with d_ctf only.
+bool lines_fits(int N, int n);
+size_t lines_edge_bytes(int N, int n);
+int launch_lines(const float *d_raw, const float *const *d_src, int n, int box, int N,
+                 const void *d_ctf, const float *d_txy, bool means, const float *d_rot,
+                 const float *d_sym, int nsym, float *d_t3d, const PartSym *d_psym,
+                 float scale_out, float *d_img, double *d_edge, float2 *d_out, cudaStream_t st);
 void ctf_constants(float defocus, float dfdiff, float dfang, float voltage, float cs, float apix,
                    float ampcont, int N, void *out);
 // The same for a particle whose other constants are those at `from`.

@@ -67,3 +67,62 @@ def test_particles_sizes(gpu, box, N):
     o.insert(sl, rots, w, "gauss_2", "c1")
     assert oracle.rel_l2(nm, o.norm) < 2e-6
     assert oracle.rel_l2(d, o.data) < RTOL
+
+
+@pytest.mark.parametrize("box,N,n", [(16, 16, 1), (13, 26, 6), (101, 150, 3), (70, 60, 2),
+                                     (200, 240, 6), (170, 242, 2), (256, 384, 1), (300, 286, 2)])
+def test_few_particles(gpu, box, N, n):
+    """A call of few particles (fr_lines.cu): one to three passes a line, odd
+    and oversized boxes, each call's particles with and without a phase flip."""
+    from eman2_b200 import Reconstructors
+    from eman2_b200.particles import particle_meta
+    from eman2_b200.synth import quaternion_blocks, random_quaternions
+    rng = np.random.default_rng(N + n)
+    for defocus in ([0.0] * n, [1.5 - 1.5 * (i % 2) for i in range(n)]):
+        img = (rng.normal(size=(n, box, box)) + 3.0).astype(np.float32)
+        rots = quaternion_blocks(random_quaternions(n, rng))
+        shifts = np.asarray([(2.25, -1.5), (0, 0), (-N, 1), (1e-7, 0), (-0.5, 3), (4, N / 2)],
+                            np.float32)[:n]
+        w = rng.uniform(0.5, 1.0, n).astype(np.float32)
+        ctf = {"dfdiff": 0.1, "dfang": 30.0}
+        r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
+        r.setup()
+        r.insert_particles(img, particle_meta(rots, shifts, w, ctf=ctf,
+                                              defocus=np.asarray(defocus, np.float32)))
+        d, nm = r.get_accumulators()
+        sl = np.stack([oracle.particle_to_slice(img[i], N, shifts[i],
+                                                dict(ctf, defocus=float(defocus[i])))
+                       for i in range(n)])
+        o = oracle.OracleVolume(N, "fp32acc64")
+        o.insert(sl, rots, w, "gauss_2", "c1")
+        assert oracle.rel_l2(nm, o.norm) < 2e-6
+        assert oracle.rel_l2(d, o.data) < RTOL
+
+
+@pytest.mark.parametrize("N,n,shift", [(32, 4, 1), (32, 64, 1), (32, 4, 0), (32, 64, 0),
+                                       (242, 2, 1), (242, 2, 0)])
+def test_slices_over_images(gpu, N, n, shift):
+    """Slices written over the memory of their own images come out as they do
+    into memory of their own."""
+    import torch
+    from eman2_b200 import Reconstructors, _lib
+    rng = np.random.default_rng(N + n)
+    img = rng.normal(size=(n, N, N)).astype(np.float32)
+    inv = rng.uniform(-5, 5, (n, 2)).astype(np.float32)
+    want = np.stack([oracle.preprocess_slice(img[i], float(inv[i, 0]), float(inv[i, 1]))
+                     for i in range(n)])
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
+    r.setup()
+    buf = torch.zeros(n * N * (N + 2) + 2, device="cuda")
+    if shift:      # images behind the slices' start, in the slices' memory
+        src = buf[2:2 + n * N * N]
+    else:
+        src = buf[:n * N * N]
+    src.copy_(torch.from_numpy(img).reshape(-1))
+    d_inv = torch.from_numpy(inv).cuda()
+    torch.cuda.synchronize()
+    _lib.check(_lib.load().fr_preprocess_slices(r.handle, src.data_ptr(), n, d_inv.data_ptr(),
+                                                buf.data_ptr()))
+    got = buf[:n * N * (N + 2)].cpu().numpy().reshape(n, N, N + 2)
+    for i in range(n):
+        assert oracle.rel_l2(got[i], want[i]) < RTOL, i
