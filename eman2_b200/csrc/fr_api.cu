@@ -420,8 +420,6 @@ InsertJob make_job(fr_recon *r, const float2 *slices, const float *t3d, const fl
   memset(&j, 0, sizeof j);   // padding too: jobs are compared bytewise for reuse
   j.data = r->vol_data.as<float>();
   j.norm = r->vol_norm.as<float>();
-  j.fdata = j.data;
-  j.fnorm = j.norm;
   j.slices = slices;
   j.t3d = t3d;
   j.pw = pw;
@@ -466,9 +464,7 @@ int run_scatter(const InsertJob &j0, bool edge_only, cudaStream_t st) {
 void PlaneBufs::ensure(int N, long slices, cudaStream_t st) {
   int half, copies;
   centre.ensure_zero(plane_centre(N, slices, half, copies), st);
-  if (plane_partial(N, slices))
-    (void)(data.ensure_zero(vol_floats(N) * sizeof(float), st) &&
-           norm.ensure_zero(norm_floats(N) * sizeof(float), st));
+  if (plane_partial(N, slices)) quad.ensure_zero(norm_floats(N) * sizeof(float4), st);
 }
 
 int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st) {
@@ -481,12 +477,8 @@ int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st) {
     j.cdata = b.centre.as<float>();
     j.centre = half;
   }
-  const bool part = plane_partial(N, slices) && b.data.cap >= vol_floats(N) * sizeof(float) &&
-                    b.norm.cap >= norm_floats(N) * sizeof(float);
-  if (part) {
-    j.data = b.data.as<float>();
-    j.norm = b.norm.as<float>();
-  }
+  const bool part = plane_partial(N, slices) && b.quad.cap >= norm_floats(N) * sizeof(float4);
+  if (part) j.quad = b.quad.as<float4>();
   const long turns = part || j.cdata ? (slices + kPlaneTurn - 1) / kPlaneTurn : 1;
   const int per = (int)((j0.np + turns - 1) / turns);
   for (int p0 = 0; p0 < j0.np; p0 += per) {
@@ -496,7 +488,7 @@ int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st) {
     j.pw = j0.pw + p0;
     CU(launch_plane(j, st));
     if (j.cdata) CU(launch_merge_centre(nullptr, 1, &j, j.mode, j.centre, st));
-    if (part) CU(launch_merge(j0.data, j0.norm, j.data, j.norm, N, j0.corners, st));
+    if (part) CU(launch_merge(j, st));
   }
   return FR_OK;
 }

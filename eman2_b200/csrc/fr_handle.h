@@ -76,11 +76,11 @@ struct ZeroBuf : DevBuf {
   }
 };
 struct PlaneBufs {
-  ZeroBuf data, norm, centre;
+  ZeroBuf quad, centre;
   // Makes room for a call (plane_partial, plane_centre decide what it uses).
   void ensure(int N, long slices, cudaStream_t st);
   void release() {
-    for (DevBuf *b : {(DevBuf *)&data, (DevBuf *)&norm, (DevBuf *)&centre}) b->release();
+    for (DevBuf *b : {(DevBuf *)&quad, (DevBuf *)&centre}) b->release();
   }
 };
 

@@ -6,6 +6,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <climits>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -37,7 +38,7 @@ extern const TileShape kTiles[kNumTiles];
 struct InsertJob {
   float *data;               // [N][N][N+2]
   float *norm;               // [N][N][N/2+1]
-  float *fdata, *fnorm;      // the accumulators, where data and norm are a partial volume
+  float4 *quad;              // partial volume, (value, weight, 0) a cell, or null (fr_plane.cu)
   const float2 *slices;      // [np][N][N/2+1]
   const float *t3d;          // [np*nsym][9]
   const float *pw;           // [np] weight per particle
@@ -166,10 +167,15 @@ inline bool plane_small(int mode, int N, long slices) {
 // many slices or more insert into a partial volume in turns of kPlaneTurn
 // slices, each added to the accumulators once (launch_merge, which clears the
 // partial volume again), so a cell's sums stay short ones however many
-// slices a job has.  The merge costs as much as about N / 4 slices' insertion,
-// whence the limit.
+// slices a job has.  A cell's value and weight lie together in it, so that
+// one reduction adds to both.  The merge costs as much as about N / 4 slices'
+// insertion, whence the limit; beyond the L2 cache, where the reductions that
+// it saves wait for memory, half of it (gauss_2, d7, N = 384: 37 particles
+// 1.61 ms with the merge, 1.74 without; 128 particles 5.1 and 6.1).
 constexpr int kPlaneTurn = 2048;
-inline bool plane_partial(int N, long slices) { return slices >= 256 && slices * 3 >= 8L * N; }
+inline bool plane_partial(int N, long slices) {
+  return slices >= 256 && slices * 3 >= (N <= 352 ? 8L : 4L) * N;
+}
 // Every slice meets the cells near the origin.  Calls of 16 slices or more
 // add them to one of several copies of that cube, about 64 slices to each,
 // summed in double afterwards (launch_merge_centre, which clears them), so
@@ -180,18 +186,20 @@ size_t plane_centre(int N, long slices, int &half, int &copies);
 // copies return; another mode's may still be inserting on another stream).
 cudaError_t launch_merge_centre(const InsertJob *d_jobs, int njobs, const InsertJob *one, int mode,
                                 int half, cudaStream_t st);
-cudaError_t launch_merge(float *data, float *norm, float *pdata, float *pnorm, int N, int corners,
-                         cudaStream_t st);
+cudaError_t launch_merge(const InsertJob &j, cudaStream_t st);
 cudaError_t launch_pixel(const InsertJob *d_jobs, const int4 *d_work, int nwork, int block,
                          int *d_counter, int maxN, cudaStream_t st);
 // The kernel a job of this mode and size runs for a requested tile id.  The
-// two-tap windows' runs are short, so beyond the L2 cache the plane-column
+// two-tap windows' runs are short, so far beyond the L2 cache the plane-column
 // kernel waits for memory on every run, while the tile kernel adds to a tile
-// many times before it flushes it: N = 288 21.6 against 26.2 us a particle
-// (gauss_2, d7), N = 384 47.6 against 45.9, N = 480 87 against 72.
+// many times before it flushes it.  gauss_2, d7, plane against tile, us a
+// particle: N = 288 21.6, 26.2; N = 384 39.7, 43.7 (37 particles 43.6, 47.0);
+// N = 480 66, 68 (32 particles 86, 75); N = 640 121, 121.  trilinear, N = 384
+// 43.1, 42.4.
 inline int effective_tile(int tile, int mode, int N) {
   if (tile != kPlaneTile && tile != kPixelTile) return tile;
-  return mode == 5 || (plane_mode(mode) && N <= 352) ? kPlaneTile : kPixelTile;
+  const int most = mode == 5 ? INT_MAX : (mode == 2 ? 432 : 352);
+  return plane_mode(mode) && N <= most ? kPlaneTile : kPixelTile;
 }
 // The kernels over 16^3 tiles and slice blocks (int4 work items).
 inline bool is_column_tile(int tile) { return tile == kColumnTile || tile == kPixelTile; }

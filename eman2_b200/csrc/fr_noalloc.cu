@@ -148,8 +148,6 @@ extern "C" int fr_insert_slices_noalloc(const float *d_slices, int n, int N, int
   memset(&j, 0, sizeof j);
   j.data = d_data;
   j.norm = d_norm;
-  j.fdata = d_data;
-  j.fnorm = d_norm;
   j.slices = reinterpret_cast<const float2 *>(d_slices);
   j.t3d = scr + kT3dOff;
   j.pw = d_weights;

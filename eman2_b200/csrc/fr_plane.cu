@@ -13,6 +13,14 @@
 // before that, so there are neither barriers nor shared-memory atomics, and a
 // warp (an 8 x 4 patch of columns) depends on no other warp.
 //
+// Reductions are free while the volume fits L2 and cost a quarter of the time
+// beyond it (gauss_2, d7, N = 384: 47.4 us a particle with two a cell, 37.0
+// with the value's alone, 34.4 with none), by the request rather than by the
+// byte.  So a large call's partial volume holds a cell's value and weight
+// together, one 16-byte reduction (39.4), and a run's cells are addressed by a
+// stride.  Walking eight neighbouring columns in step, which puts their
+// reductions into one line, took more instructions than it saved (45.0).
+//
 // What bounds it: issue slots (76 % of cycles issue at gauss_5, 75 % at
 // gauss_2 while the volume fits L2), at 69 % of lanes busy: the windows of a
 // warp's columns hold unequal pixel counts.  A gauss_5 tap takes 36 thread
@@ -20,9 +28,9 @@
 // six taps, the weights go through packed operations, and a cell leaves the
 // registers once.
 // Measured on one B200, insertion alone (the kernels it took over from in
-// parentheses): gauss_5, d7, N = 384, 64 particles 20.1 ms (46.8, tile columns
+// parentheses): gauss_5, d7, N = 384, 64 particles 19.5 ms (46.8, tile columns
 // with shared read-modify-writes), one particle 0.43 ms (1.32, an atomic per
-// tap); gauss_2, c1, N = 192, 2048 particles 1.52 ms (2.12, tiles with shared
+// tap); gauss_2, c1, N = 192, 2048 particles 1.46 ms (2.12, tiles with shared
 // atomics).  Blocks an SM: gauss_5 without spills (two of eight warps, 128
 // registers) against three at 80, 20.1 against 21.6 ms; five or four of four
 // warps 20.8 and 20.3.  The two-tap windows at three blocks 1.52 ms, two 1.70,
@@ -171,6 +179,28 @@ __device__ __forceinline__ int centre_cell(int c, int i, int j, int l) {
   return ((l + c) * (2 * c + 1) + j + c) * (c + 1) + i;
 }
 
+// add_tap_atomic's placement rules in a partial volume; launch_merge keeps the
+// imaginary parts of the two self-conjugate cells zero.
+__device__ __forceinline__ void quad_tap(float4 *quad, int N, int x, int y, int z, float re,
+                                         float im, float w) {
+  const int h = N >> 1, w2 = h + 1;
+  if (abs(x) > h || abs(y) > h || abs(z) > h) return;
+  float4 *mirror = quad + (size_t)((y <= 0 ? -y : N - y) + (z <= 0 ? -z : N - z) * N) * w2 + abs(x);
+  if (x == 0 || abs(x) == h) {
+    if (y == 0 && z == 0) {
+      atomicAdd(mirror, make_float4(re, 0.0f, w, 0.0f));
+      return;
+    }
+    atomicAdd(mirror, make_float4(re, -im, 0.0f, 0.0f));
+  }
+  if (x < 0) {
+    atomicAdd(mirror, make_float4(re, -im, w, 0.0f));
+    return;
+  }
+  atomicAdd(quad + (size_t)((y < 0 ? N + y : y) + (z < 0 ? N + z : z) * N) * w2 + x,
+            make_float4(re, im, w, 0.0f));
+}
+
 // Adds the sums of tap cell (i, j, l) of a slice to the volume, or to the
 // slice's copy of the cells near the origin (see plane_centre).
 __device__ __forceinline__ void place(const InsertJob &J, float2 *cd, float *cn, int i, int j, int l,
@@ -185,6 +215,8 @@ __device__ __forceinline__ void place(const InsertJob &J, float2 *cd, float *cn,
       if (!origin) atomicAdd(cd + centre_cell(c, 0, -j, -l), make_float2(re, -im));
       atomicAdd(cd + at, make_float2(re, origin ? 0.0f : im));
       atomicAdd(cn + at, w);
+    } else if (J.quad) {
+      quad_tap(J.quad, N, i, j, l, re, im, w);
     } else {
       add_tap_atomic(J.data, J.norm, N, N, i, j, l, re, im, w);
     }
@@ -207,6 +239,10 @@ __device__ __forceinline__ void place(const InsertJob &J, float2 *cd, float *cn,
     norm = cn;
   } else {
     at = (size_t)ia + (size_t)((j < 0 ? N + j : j) + (l < 0 ? N + l : l) * N) * w2;
+    if (J.quad) {
+      atomicAdd(J.quad + at, make_float4(re, im, w, 0.0f));
+      return;
+    }
   }
   atomicAdd(data + at, make_float2(re, im));
   atomicAdd(norm + at, w);
@@ -372,6 +408,49 @@ __device__ __forceinline__ void column(const InsertJob &J, const Smem &S, int A,
   }
   // the run into the volume; its words go back to zero for the next column
   const float wscale = MODE == MODE_TRILINEAR ? 1.0f : w;
+  // Most runs stay clear of the planes x = 0 and N/2, of the row or slab where
+  // indices wrap and of the centre copies: their cells are one stride apart,
+  // and a run below x = 0 goes to its mirror cells, conjugated.
+  const int ke = kb + nq - 1, reach = max(abs(tb), abs(tc)), side = A == 0 ? kb : tb;
+  const int centre = cd ? J.centre : -1;
+  if (max(reach, max(abs(kb), abs(ke))) < n2 && (kb > 0 || ke < 0) && side != 0 &&
+      !(reach <= centre && min(abs(kb), abs(ke)) <= centre)) {
+    const int sg = side < 0 ? -1 : 1;
+    const int i = sg * side, j = sg * (A == 1 ? kb : (A == 0 ? tb : tc)), l = sg * (A == 2 ? kb : tc);
+    const size_t at = (size_t)i + (size_t)((j < 0 ? N + j : j) + (l < 0 ? N + l : l) * N) * w2;
+    const int step = sg * (A == 0 ? 1 : (A == 1 ? w2 : w2 * N));
+    const float sgf = (float)sg;
+    if (J.quad) {   // one reduction a cell
+      float4 *pq = J.quad + at;
+      float2 *pv = S.sv + lane;
+      float *pw = S.sw + lane;
+#pragma unroll 1
+      for (int q = 0; q < nq; q++, pq += step, pv += 32, pw += 32) {
+        const float2 v = *pv;
+        const float s = *pw;
+        if (v.x == 0.0f && v.y == 0.0f && s == 0.0f) continue;
+        *pv = make_float2(0.0f, 0.0f);
+        *pw = 0.0f;
+        atomicAdd(pq, make_float4(v.x, sgf * v.y, s * wscale, 0.0f));
+      }
+      return;
+    }
+    float2 *pd = reinterpret_cast<float2 *>(J.data) + at;
+    float *pn = J.norm + at;
+    float2 *pv = S.sv + lane;
+    float *pw = S.sw + lane;
+#pragma unroll 1
+    for (int q = 0; q < nq; q++, pd += step, pn += step, pv += 32, pw += 32) {
+      const float2 v = *pv;
+      const float s = *pw;
+      if (v.x == 0.0f && v.y == 0.0f && s == 0.0f) continue;
+      *pv = make_float2(0.0f, 0.0f);
+      *pw = 0.0f;
+      atomicAdd(pd, make_float2(v.x, sgf * v.y));
+      atomicAdd(pn, s * wscale);
+    }
+    return;
+  }
 #pragma unroll 1
   for (int q = 0; q < nq; q++) {
     const int at = q * 32 + lane;
@@ -430,7 +509,7 @@ __device__ __forceinline__ void slice_part(const InsertJob &J, const Smem &S, in
       float xx, yy, zz;
       pixel_coords(S.rtab[x + n2], S.rtab[y + n2], M, (float)N, xx, yy, zz);
       const float2 v = slice_value(sl, N, x, y);
-      insert_pixel_atomic<MODE>(J.fdata, J.fnorm, N, N, xx, yy, zz, v.x, v.y, w, h, table, false);
+      insert_pixel_atomic<MODE>(J.data, J.norm, N, N, xx, yy, zz, v.x, v.y, w, h, table, false);
     }
     return;
   }
@@ -598,8 +677,8 @@ __global__ void __launch_bounds__(plane::Win<MODE>::NT, plane::Win<MODE>::CTAS)
 // per row; cells farther than the pixels and their windows reach are skipped.
 // The two self-conjugate cells keep a zero imaginary part once touched.
 __global__ void __launch_bounds__(128)
-    k_merge(float2 *__restrict__ data, float *__restrict__ norm, float2 *__restrict__ pdata,
-            float *__restrict__ pnorm, int N, float reach) {
+    k_merge(float2 *__restrict__ data, float *__restrict__ norm, float4 *__restrict__ quad, int N,
+            float reach) {
   const int w2 = N / 2 + 1;
   const int y = blockIdx.x, z = blockIdx.y;
   const float fy = (float)(y <= N / 2 ? y : y - N), fz = (float)(z <= N / 2 ? z : z - N);
@@ -608,18 +687,16 @@ __global__ void __launch_bounds__(128)
   const int n = min(w2, (int)sqrtf(left) + 2);
   const size_t row = ((size_t)z * N + y) * w2;
   for (int x = threadIdx.x; x < n; x += blockDim.x) {
-    const float s = pnorm[row + x];
-    const float2 v = pdata[row + x];
+    const float4 v = quad[row + x];
     // (an x = 0 cell may hold conjugate values and no weight)
-    if (s == 0.0f && v.x == 0.0f && v.y == 0.0f) continue;
+    if (v.z == 0.0f && v.x == 0.0f && v.y == 0.0f) continue;
     float2 d = data[row + x];
     d.x += v.x;
     d.y += v.y;
     if (y == 0 && z == 0 && (x == 0 || x == w2 - 1)) d.y = 0.0f;
     data[row + x] = d;
-    norm[row + x] += s;
-    pdata[row + x] = make_float2(0.0f, 0.0f);
-    pnorm[row + x] = 0.0f;
+    norm[row + x] += v.z;
+    quad[row + x] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
 }
 
@@ -651,12 +728,12 @@ __global__ void __launch_bounds__(256)
   if (!any) return;
   const int i = q % (c + 1), j = (q / (c + 1)) % side - c, l = q / ((c + 1) * side) - c;
   const size_t at = (size_t)i + (size_t)((j < 0 ? N + j : j) + (l < 0 ? N + l : l) * N) * w2;
-  float2 *d = reinterpret_cast<float2 *>(J.fdata) + at;
+  float2 *d = reinterpret_cast<float2 *>(J.data) + at;
   float2 v = *d;
   v.x += (float)re;
   v.y = (i == 0 && j == 0 && l == 0) ? 0.0f : v.y + (float)im;
   *d = v;
-  J.fnorm[at] += (float)w;
+  J.norm[at] += (float)w;
 }
 
 static int plane_parts(int N, int mode, long slices) {
@@ -773,14 +850,13 @@ cudaError_t launch_merge_centre(const InsertJob *d_jobs, int njobs, const Insert
   return cudaGetLastError();
 }
 
-cudaError_t launch_merge(float *data, float *norm, float *pdata, float *pnorm, int N, int corners,
-                         cudaStream_t st) {
+cudaError_t launch_merge(const InsertJob &j, cudaStream_t st) {
   // the farthest pixel (the kernel takes matrices within 1 % of a rotation)
   // and the corner of its window
-  const float reach = 1.01f * (corners ? 0.7072f * N + 1.0f : 0.5f * N + 0.52f) + 3.5f * 1.7321f;
+  const float reach = 1.01f * (j.corners ? 0.7072f * j.N + 1.0f : 0.5f * j.N + 0.52f) + 3.5f * 1.7321f;
   note_launch();
-  k_merge<<<dim3(N, N), 128, 0, st>>>(reinterpret_cast<float2 *>(data), norm,
-                                      reinterpret_cast<float2 *>(pdata), pnorm, N, reach);
+  k_merge<<<dim3(j.N, j.N), 128, 0, st>>>(reinterpret_cast<float2 *>(j.data), j.norm, j.quad, j.N,
+                                          reach);
   return cudaGetLastError();
 }
 
