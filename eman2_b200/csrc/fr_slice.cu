@@ -254,8 +254,13 @@ template <int DIR> __device__ void split_rows(float2 *z, const Shape &s, const C
   }
 }
 
+// R1's cases.  17 and 19 have a kernel of their own (BIG): with them among the
+// others those took more registers (N = 240, 600 particles 656 against 637 us).
 #define FR_RADIX(R, CALL)             \
-  switch (R) {                        \
+  if constexpr (BIG) {                \
+    if (R == 17) CALL(17);            \
+    else CALL(19);                    \
+  } else switch (R) {                 \
     case 2: CALL(2); break;           \
     case 3: CALL(3); break;           \
     case 4: CALL(4); break;           \
@@ -265,7 +270,9 @@ template <int DIR> __device__ void split_rows(float2 *z, const Shape &s, const C
     case 8: CALL(8); break;           \
     case 9: CALL(9); break;           \
     case 10: CALL(10); break;         \
+    case 11: CALL(11); break;         \
     case 12: CALL(12); break;         \
+    case 13: CALL(13); break;         \
     case 14: CALL(14); break;         \
     case 15: CALL(15); break;         \
     default: CALL(16); break;         \
@@ -283,6 +290,7 @@ template <int DIR> __device__ void split_rows(float2 *z, const Shape &s, const C
   }
 
 // Image -> half spectrum, last column pass left to the caller.
+template <bool BIG>
 __device__ __forceinline__ void forward(float2 *z, const Shape &s, const Cols &t) {
 #define CALL(R) row_outer<R, -1>(z, s, 1.0f)
   FR_RADIX(s.R1, CALL)
@@ -424,7 +432,7 @@ struct Args {
 
 }  // namespace slc
 
-__global__ void __launch_bounds__(768, 1) k_slice(slc::Args a, slc::Shape s) {
+template <bool BIG> __global__ void __launch_bounds__(768, 1) k_slice(slc::Args a, slc::Shape s) {
   using namespace slc;
   extern __shared__ __align__(16) unsigned char dyn[];
   const int N = s.N, n2 = N / 2, box = a.box, p = blockIdx.x;
@@ -486,7 +494,7 @@ __global__ void __launch_bounds__(768, 1) k_slice(slc::Args a, slc::Shape s) {
   if (a.ctf && a.ctf[p].on != 0.0f) {
     const CtfDev ctf = a.ctf[p];
     const float scale_in = 1.0f / ((float)N * (float)N);   // do_ift's
-    forward(z, s, t);
+    forward<BIG>(z, s, t);
 #define CALL(R) col_inner<R, 1>(z, s, t, &ctf)
     FR_EVEN_RADIX(s.R2, CALL)
 #undef CALL
@@ -521,7 +529,7 @@ __global__ void __launch_bounds__(768, 1) k_slice(slc::Args a, slc::Shape s) {
   }
   translate(z, s, a.txy ? a.txy[2 * (size_t)p] : 0.0f, a.txy ? a.txy[2 * (size_t)p + 1] : 0.0f,
             mean, a.scale_out);
-  forward(z, s, t);
+  forward<BIG>(z, s, t);
 #define CALL(R) col_inner<R, 0>(z, s, t, nullptr)
   FR_EVEN_RADIX(s.R2, CALL)
 #undef CALL
@@ -536,11 +544,11 @@ static size_t slice_smem(int N) {
 }
 static bool slice_radices(int N, int &R1, int &R2) {
   if (N < 16 || slice_smem(N) > 232448) return false;
-  const int all[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16};
+  const int all[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 19};
   int best = 1 << 30;
   for (int a : all)
     for (int b : all) {
-      if (a * b != N || b % 2) continue;
+      if (a * b != N || b % 2 || b > 16) continue;
       const int worst = std::max(a, b);
       if (worst < best || (worst == best && b < R2)) {
         best = worst;
@@ -550,14 +558,17 @@ static bool slice_radices(int N, int &R1, int &R2) {
     }
   return best < (1 << 30);
 }
-// A block takes 26 us (N = 96, no CTF) to 87 us (N = 192, CTF) for its
-// particle, as long as the separate launches take for a few dozen; with the
-// CTF's extra launches those lose from the first particle at the small sizes
-// (one particle, N = 96: 73 us a call against 81; N = 192: 105 against 77, 148
-// particles 119 against 284).
+// A block takes its particle 26 us (N = 96, no CTF) to 87 us (N = 192, CTF),
+// however few there are, where the line preparation takes 28 to 46 us for up to
+// a dozen.  With a CTF, us a call, against it: N = 88, 1 particle 44, 44; N =
+// 112, 1 55, 46; N = 96, 16 53, 45 and 24 53, 67; N = 144, 48 75, 68 and 64
+// 102, 105; N = 192, 64 115, 132.  Against the library's transforms (sizes with
+// a radix of 17 or 19): N = 152, 1 85, 50 and 48 90, 128.
 bool slice_fits(int N, int n, bool ctf) {
   int a = 0, b = 0;
-  return (n >= 48 || (ctf && N <= 112)) && slice_radices(N, a, b);
+  if (!slice_radices(N, a, b)) return false;
+  if (std::max(a, b) > 16) return n >= 24;
+  return n >= 56 || (ctf && (N <= 88 || (N <= 112 && n >= 20)));
 }
 // Threads of a block: several blocks share an SM at the smaller sizes
 // (2,000 particles: N = 96 0.33, 0.37, 0.48 ms with 256, 384, 768 threads;
@@ -618,9 +629,10 @@ int launch_slice(const float *d_raw, const float *const *d_src, int n, int box, 
   a.scale_out = scale_out;
   a.out = d_out;
   const size_t smem = slice_smem(N);
-  CU(set_max_smem((const void *)k_slice, smem));
+  auto *kernel = s.R1 > 16 ? k_slice<true> : k_slice<false>;
+  CU(set_max_smem((const void *)kernel, smem));
   note_launch();
-  k_slice<<<n, slice_threads(N), smem, st>>>(a, s);
+  kernel<<<n, slice_threads(N), smem, st>>>(a, s);
   CU(cudaGetLastError());
   return FR_OK;
 }

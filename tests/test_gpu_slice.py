@@ -22,10 +22,10 @@ def _shifts(n, N, rng):
     return s
 
 
-@pytest.mark.parametrize("N", [16, 18, 30, 42, 84, 98, 150, 196, 240])
+@pytest.mark.parametrize("N", [16, 18, 30, 42, 76, 84, 98, 150, 170, 196, 208, 240])
 def test_preprocess_sizes(gpu, N):
     from eman2_b200 import Reconstructors, _lib
-    n = 48
+    n = 56
     rng = np.random.default_rng(N)
     img = rng.normal(size=(n, N, N)).astype(np.float32)
     inv = _shifts(n, N, rng)
@@ -43,7 +43,7 @@ def test_preprocess_sizes(gpu, N):
 
 
 @pytest.mark.parametrize("box,N", [(11, 16), (64, 96), (101, 150), (33, 32), (70, 60), (128, 192),
-                                   (160, 240)])
+                                   (101, 152), (120, 176), (160, 240)])
 def test_particles_sizes(gpu, box, N):
     from eman2_b200 import Reconstructors
     from eman2_b200.particles import particle_meta
@@ -56,6 +56,8 @@ def test_particles_sizes(gpu, box, N):
     w = rng.uniform(0.5, 1.0, n).astype(np.float32)
     df = rng.uniform(0.8, 2.5, n).astype(np.float32)
     df[::5] = 0.0
+    take = np.arange(56) % n   # as many as the one launch asks for
+    n, img, rots, shifts, w, df = 56, img[take], rots[take], shifts[take], w[take], df[take]
     ctf = {"dfdiff": 0.1, "dfang": 30.0}
     r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
     r.setup()
@@ -70,7 +72,8 @@ def test_particles_sizes(gpu, box, N):
 
 
 @pytest.mark.parametrize("box,N,n", [(16, 16, 1), (13, 26, 6), (101, 150, 3), (70, 60, 2),
-                                     (200, 240, 6), (170, 242, 2), (256, 384, 1), (300, 286, 2)])
+                                     (200, 240, 6), (170, 242, 2), (256, 384, 1), (300, 286, 2),
+                                     (150, 224, 40), (90, 252, 47)])
 def test_few_particles(gpu, box, N, n):
     """A call of few particles (fr_lines.cu): one to three passes a line, odd
     and oversized boxes, each call's particles with and without a phase flip."""
@@ -81,8 +84,9 @@ def test_few_particles(gpu, box, N, n):
     for defocus in ([0.0] * n, [1.5 - 1.5 * (i % 2) for i in range(n)]):
         img = (rng.normal(size=(n, box, box)) + 3.0).astype(np.float32)
         rots = quaternion_blocks(random_quaternions(n, rng))
-        shifts = np.asarray([(2.25, -1.5), (0, 0), (-N, 1), (1e-7, 0), (-0.5, 3), (4, N / 2)],
-                            np.float32)[:n]
+        shifts = rng.uniform(-5, 5, (n, 2)).astype(np.float32)
+        fixed = [(2.25, -1.5), (0, 0), (-N, 1), (1e-7, 0), (-0.5, 3), (4, N / 2)][:n]
+        shifts[:len(fixed)] = fixed
         w = rng.uniform(0.5, 1.0, n).astype(np.float32)
         ctf = {"dfdiff": 0.1, "dfang": 30.0}
         r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
