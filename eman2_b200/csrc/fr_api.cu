@@ -735,7 +735,7 @@ int prologue_run(PlanCache &plans, const ProScratch &b, const unsigned char *d_m
   if (slice_fits(N, n, any_ctf))
     return launch_slice(d_raw, d_src, n, box, N, any_ctf ? mv.ctf : nullptr, mv.txy, true, mv.rot,
                         d_sym, nsym, b.t3d->as<float>(), d_psym, scale, b.slices->as<float2>(), st);
-  if (lines_fits(N, n)) {
+  if (lines_fits(N, n, any_ctf)) {
     if (any_ctf) {
       TRY(b.img->ensure(sizeof(float) * img * n));
       TRY(b.spec->ensure(lines_edge_bytes(N, n)));
@@ -1016,7 +1016,7 @@ static int preprocess_device(fr_recon *r, const float *d_imgs, int n, const floa
   if (direct && slice_fits(N, n, false))
     return launch_slice(d_imgs, nullptr, n, N, N, nullptr, d_txy, false, nullptr, nullptr, 0,
                         nullptr, nullptr, scale, (float2 *)d_out_slices, st);
-  if (direct && lines_fits(N, n))
+  if (direct && lines_fits(N, n, false))
     return launch_lines(d_imgs, nullptr, n, N, N, nullptr, d_txy, false, nullptr, nullptr, 0,
                         nullptr, nullptr, scale, nullptr, nullptr, (float2 *)d_out_slices, st);
   TRY(r->s_img2.ensure(sizeof(float) * (size_t)n * N * N));

@@ -222,8 +222,8 @@ cudaError_t launch_pad_compose(const float *d_raw, const float *const *d_src, in
                                float *d_img, const float *d_rot, const float *d_sym, int nsym,
                                float *d_t3d, cudaStream_t st, const PartSym *d_psym = nullptr);
 // The whole preparation of n particles in one launch (fr_slice.cu), where
-// slice_fits says that it is possible and the better way.  d_ctf, d_txy, d_rot null: no phase flip, no shift,
-// no composition; means: subtract the edge means.
+// slice_fits says that it is possible and the better way.  d_ctf, d_txy, d_rot
+// null: no phase flip, no shift, no composition; means: subtract the edge means.
 bool slice_fits(int N, int n, bool ctf);
 int launch_slice(const float *d_raw, const float *const *d_src, int n, int box, int N,
                  const void *d_ctf, const float *d_txy, bool means, const float *d_rot,
@@ -231,7 +231,7 @@ int launch_slice(const float *d_raw, const float *const *d_src, int n, int box, 
                  float scale_out, float2 *d_out, cudaStream_t st);
 // The same in up to five launches (fr_lines.cu), where lines_fits says so;
 // d_img, d_edge: n images and lines_edge_bytes of workspace, with d_ctf only.
-bool lines_fits(int N, int n);
+bool lines_fits(int N, int n, bool ctf);
 size_t lines_edge_bytes(int N, int n);
 int launch_lines(const float *d_raw, const float *const *d_src, int n, int box, int N,
                  const void *d_ctf, const float *d_txy, bool means, const float *d_rot,

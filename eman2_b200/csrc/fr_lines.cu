@@ -1,6 +1,7 @@
 // fr_lines.cu -- the per-particle preparation as five launches over lines (rows
-// or columns) of every particle, for calls of few particles (fr_slice.cu gives
-// a block a whole particle, which pays from some tens of particles on).
+// or columns) of every particle: calls of few particles, and images larger
+// than one SM's shared memory (fr_slice.cu gives a block a whole particle,
+// which pays from some tens of particles on).
 //
 //   rows:    edge mean, zero-padded clip, FFT along x          (CTF particles)
 //   columns: FFT along y, CTF sign, FFT back                   (CTF particles)
@@ -8,14 +9,21 @@
 //   rows:    edge mean, bilinear shift, FFT along x
 //   columns: FFT along y, phase origin to corner, the slice
 //
-// A block takes a few lines into shared memory, transforms them there and
-// writes them out, so a stage reads and writes its image once; the half spectra
-// live in the slices' own buffer.  Two real rows make one complex line.  What
-// bounds it: launch latency, and each block's load, few dependent passes and
-// store, some 8 us a stage however little there is to do.  That is why the
-// stages are five and not ten, and why a block has as few as two lines: one
-// particle with a CTF at N = 192 47 us (62 in ten launches with the library's
-// transforms, two of which are its own rows and columns), N = 384 55 (59).
+// A block takes up to sixteen lines (128 bytes of a row) into shared memory,
+// transforms them there and writes them out, so a stage reads and writes its
+// image once; the half spectra live in the slices' own buffer.  Two real rows
+// make one complex line.
+//
+// What bounds it: for one particle, launches and each block's load, two or
+// three dependent passes and store, some 8 us a stage however little there is
+// to do; that is why the stages are five and not ten, why a block then has as
+// few as two lines, and why a stage's blocks start while the one before it
+// drains.  For many, instructions (56 % of cycles issue) at four blocks an SM.
+// A call with a CTF, against the ten launches with the library's transforms
+// (fr_prologue.cu), us: N = 192, 1 particle 46 (62), 16 61 (73); N = 256, 128
+// particles 224 (249); N = 384, 1 47 (60), 64 287 (373), 512 1930 (2420); N =
+// 480, 512 3416 (3611).  Three blocks an SM and eight lines a block: N = 384,
+// 512 2199; loads one at a time: 3305.
 //
 // The line FFT: up to three passes of radices in registers, decimation in
 // frequency, in place: pass i takes blocks of L = R M points, butterflies over
@@ -66,6 +74,26 @@ struct Walk {
     }
   }
 };
+
+// store(slow, fast, load(slow, fast)) over w's pairs, slow < count, U loads at
+// a time: one by one each would wait for memory.
+template <int U, class L, class S>
+__device__ __forceinline__ void batched(Walk w, int count, L load, S store) {
+  while (w.slow < count) {
+    int f[U], s[U];
+    float2 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      f[u] = w.fast;
+      s[u] = w.slow;
+      v[u] = load(min(s[u], count - 1), f[u]);
+      w.next();
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (s[u] < count) store(s[u], f[u], v[u]);
+  }
+}
 
 // Pass i of `count` lines.
 template <int R, int DIR>
@@ -203,32 +231,58 @@ __device__ __forceinline__ Padded padded(const Args &a, int N, int p, double *s_
 }
 
 // Bilinear translation (TransformProcessor::transform, 2-D real branch,
-// libEM/processor.cpp:11025-11080) of at - mean, times scale: one output.
+// libEM/processor.cpp:11025-11080) of at - mean, times scale: the part that
+// one column's outputs share, then one output.
+struct Shift {
+  float tx, ty, mean, scale;
+  int N;
+  bool copy;   // Transform::is_identity
+};
+struct Column {
+  int ix, jx;
+  float t, omt;
+  bool in;
+};
+__device__ __forceinline__ Column column_of(const Shift &c, int x) {
+  const int h = c.N / 2;
+  const float x2 = __fadd_rn(__fadd_rn((float)(x - h), c.tx), (float)h);
+  Column k;
+  k.in = x2 >= 0 && x2 < c.N;
+  k.ix = c.copy ? x : k.in ? (int)x2 : 0;
+  k.jx = k.ix == c.N - 1 ? k.ix : k.ix + 1;
+  k.t = __fsub_rn(x2, (float)k.ix);
+  k.omt = __fsub_rn(1.0f, k.t);
+  return k;
+}
 template <class F>
-__device__ __forceinline__ float shifted(const F &at, int N, int y, int x, float tx, float ty,
-                                         bool copy, float mean, float scale) {
-  if (copy) return __fmul_rn(__fsub_rn(at(y, x), mean), scale);   // Transform::is_identity
-  const int h = N / 2;
-  const float x2 = __fadd_rn(__fadd_rn((float)(x - h), tx), (float)h);
-  const float y2 = __fadd_rn(__fadd_rn((float)(y - h), ty), (float)h);
-  if (!(x2 >= 0 && x2 < N && y2 >= 0 && y2 < N)) return 0.0f;
-  const int ix = (int)x2, iy = (int)y2;
-  const int jx = ix == N - 1 ? ix : ix + 1, jy = iy == N - 1 ? iy : iy + 1;
-  const float t = __fsub_rn(x2, (float)ix), u = __fsub_rn(y2, (float)iy);
-  const float omt = __fsub_rn(1.0f, t), omu = __fsub_rn(1.0f, u);
-  float v = __fmul_rn(__fmul_rn(omt, omu), __fsub_rn(at(iy, ix), mean));
-  v = __fadd_rn(v, __fmul_rn(__fmul_rn(t, omu), __fsub_rn(at(iy, jx), mean)));
-  v = __fadd_rn(v, __fmul_rn(__fmul_rn(omt, u), __fsub_rn(at(jy, ix), mean)));
-  v = __fadd_rn(v, __fmul_rn(__fmul_rn(t, u), __fsub_rn(at(jy, jx), mean)));
-  return __fmul_rn(v, scale);
+__device__ __forceinline__ float shifted(const F &at, const Shift &c, const Column &k, int y) {
+  if (c.copy) return __fmul_rn(__fsub_rn(at(y, k.ix), c.mean), c.scale);
+  const int h = c.N / 2;
+  const float y2 = __fadd_rn(__fadd_rn((float)(y - h), c.ty), (float)h);
+  // outside: 0, after loads that wait for no test
+  const bool in = k.in && y2 >= 0 && y2 < c.N;
+  const int iy = in ? (int)y2 : 0, jy = iy == c.N - 1 ? iy : iy + 1;
+  const float u = __fsub_rn(y2, (float)iy), omu = __fsub_rn(1.0f, u);
+  const float a = at(iy, k.ix), b = at(iy, k.jx), d = at(jy, k.ix), e = at(jy, k.jx);
+  float v = __fmul_rn(__fmul_rn(k.omt, omu), __fsub_rn(a, c.mean));
+  v = __fadd_rn(v, __fmul_rn(__fmul_rn(k.t, omu), __fsub_rn(b, c.mean)));
+  v = __fadd_rn(v, __fmul_rn(__fmul_rn(k.omt, u), __fsub_rn(d, c.mean)));
+  v = __fadd_rn(v, __fmul_rn(__fmul_rn(k.t, u), __fsub_rn(e, c.mean)));
+  return in ? __fmul_rn(v, c.scale) : 0.0f;
 }
 
 extern __shared__ __align__(16) unsigned char dyn[];
 
-// Shared memory: the lines, then the position table.
-__device__ __forceinline__ unsigned short *load_pos(float2 *z, int count, const Plan &p) {
+// What a stage can do before the stage it reads has finished: lets the next
+// one start, takes the position table (behind the lines in shared memory),
+// has the twiddles fetched.  Then waits for the stage before.
+__device__ __forceinline__ unsigned short *begin(float2 *z, int count, const Plan &p) {
+  cudaTriggerProgrammaticLaunchCompletion();
   unsigned short *pos = reinterpret_cast<unsigned short *>(z + count * p.ld);
   for (int i = threadIdx.x; i < p.N; i += blockDim.x) pos[i] = __ldg(&p.pos[i]);
+  for (int i = 16 * threadIdx.x; i < p.N; i += 16 * blockDim.x)
+    asm volatile("{.reg .f32 x;\n ld.global.nc.f32 x, [%0];}" ::"l"(p.tw + i));
+  cudaGridDependencySynchronize();
   return pos;
 }
 
@@ -249,33 +303,34 @@ __device__ __forceinline__ void rows_out(float2 *z, int count, int j0, const Pla
 }
 
 // First rows of the phase flip.
-__global__ void __launch_bounds__(256) k_rows_pad(Args a, Plan p, int per) {
+__global__ void __launch_bounds__(256, 4) k_rows_pad(Args a, Plan p, int per) {
   __shared__ double s_red[8];
   const int q = blockIdx.x, N = p.N, j0 = blockIdx.y * per, count = min(per, N / 2 - j0);
   if (!has_ctf(a, q)) return;
   float2 *z = reinterpret_cast<float2 *>(dyn);
-  const unsigned short *pos = load_pos(z, per, p);
+  const unsigned short *pos = begin(z, per, p);
   // rows outside the box are zero whatever its edge mean
   const int o = (a.box - N) >= 0 ? (a.box - N) / 2 : -((N - a.box + 1) / 2);
   const bool blank = 2 * (j0 + count) + o <= 0 || 2 * j0 + o >= a.box;
   const Padded at = padded(a, N, q, s_red, a.means && !blank);
-  for (Walk w(N); w.slow < count; w.next()) {
-    const int y = 2 * (j0 + w.slow);
-    z[w.slow * p.ld + pad(w.fast)] = make_float2(at(y, w.fast), at(y + 1, w.fast));
-  }
+  batched<4>(
+      Walk(N), count,
+      [&](int s, int x) { return make_float2(at(2 * (j0 + s), x), at(2 * (j0 + s) + 1, x)); },
+      [&](int s, int x, float2 v) { z[s * p.ld + pad(x)] = v; });
   rows_out(z, count, j0, p, pos, a.spec + (size_t)q * N * (N / 2 + 1));
 }
 
 // Columns there and back with the CTF's sign between.
-__global__ void __launch_bounds__(256) k_cols_flip(Args a, Plan p, int per) {
+__global__ void __launch_bounds__(256, 4) k_cols_flip(Args a, Plan p, int per) {
   const int q = blockIdx.x, N = p.N, w2 = N / 2 + 1, c0 = blockIdx.y * per,
             count = min(per, w2 - c0);
   if (!has_ctf(a, q)) return;
   float2 *z = reinterpret_cast<float2 *>(dyn);
-  const unsigned short *pos = load_pos(z, per, p);
+  const unsigned short *pos = begin(z, per, p);
   float2 *spec = a.spec + (size_t)q * N * w2 + c0;
-  for (Walk w(count); w.slow < N; w.next())
-    z[w.fast * p.ld + pad(w.slow)] = spec[(size_t)w.slow * w2 + w.fast];
+  batched<8>(
+      Walk(count), N, [&](int y, int c) { return spec[(size_t)y * w2 + c]; },
+      [&](int y, int c, float2 v) { z[c * p.ld + pad(y)] = v; });
   transform<-1>(z, count, p);
   const CtfDev k = a.ctf[q];
   for (Walk w(N); w.slow < count; w.next()) {
@@ -289,25 +344,39 @@ __global__ void __launch_bounds__(256) k_cols_flip(Args a, Plan p, int per) {
 }
 
 // Rows back to the image, scaled as do_ift scales it.
-__global__ void __launch_bounds__(256) k_rows_back(Args a, Plan p, int per) {
+__global__ void __launch_bounds__(256, 4) k_rows_back(Args a, Plan p, int per) {
   __shared__ double s_red[8];
   const int q = blockIdx.x, N = p.N, n2 = N / 2, w2 = n2 + 1, j0 = blockIdx.y * per,
             count = min(per, n2 - j0);
   if (!has_ctf(a, q)) return;
   float2 *z = reinterpret_cast<float2 *>(dyn);
-  const unsigned short *pos = load_pos(z, per, p);
+  const unsigned short *pos = begin(z, per, p);
   const float2 *spec = a.spec + (size_t)q * N * w2;
   __syncthreads();
-  for (Walk w(w2); w.slow < count; w.next()) {
-    const int k = w.fast;
-    const float2 *r = spec + (size_t)(2 * (j0 + w.slow)) * w2 + k;
-    const float2 u = r[0], v = r[w2];
-    float2 *o = z + w.slow * p.ld;
-    if (k == 0 || k == n2) {   // real along the row: an inverse real FFT reads no more
-      o[pad(pos[k])] = make_float2(u.x, v.x);
-    } else {
-      o[pad(pos[k])] = make_float2(u.x - v.y, u.y + v.x);
-      o[pad(pos[N - k])] = make_float2(u.x + v.y, v.x - u.y);
+  for (Walk w(w2); w.slow < count;) {
+    float2 us[4], vs[4];
+    int ks[4], rows[4];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      ks[g] = w.fast;
+      rows[g] = w.slow;
+      const float2 *r = spec + (size_t)(2 * (j0 + min(w.slow, count - 1))) * w2 + w.fast;
+      us[g] = r[0];
+      vs[g] = r[w2];
+      w.next();
+    }
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      if (rows[g] >= count) break;
+      const int k = ks[g];
+      const float2 u = us[g], v = vs[g];
+      float2 *o = z + rows[g] * p.ld;
+      if (k == 0 || k == n2) {   // real along the row: an inverse real FFT reads no more
+        o[pad(pos[k])] = make_float2(u.x, v.x);
+      } else {
+        o[pad(pos[k])] = make_float2(u.x - v.y, u.y + v.x);
+        o[pad(pos[N - k])] = make_float2(u.x + v.y, v.x - u.y);
+      }
     }
   }
   transform<1>(z, count, p);
@@ -330,7 +399,7 @@ __global__ void __launch_bounds__(256) k_rows_back(Args a, Plan p, int per) {
 }
 
 // Rows of the shifted image (or, without a phase flip, of the padded raw one).
-__global__ void __launch_bounds__(256) k_rows_shift(Args a, Plan p, int per) {
+__global__ void __launch_bounds__(256, 4) k_rows_shift(Args a, Plan p, int per) {
   __shared__ double s_red[8];
   const int q = blockIdx.x, N = p.N, j0 = blockIdx.y * per, count = min(per, N / 2 - j0);
   if (a.rot && blockIdx.y == 0) {   // the particle's symmetry copies (libEM/transform.cpp:1384-1395)
@@ -347,21 +416,42 @@ __global__ void __launch_bounds__(256) k_rows_shift(Args a, Plan p, int per) {
       a.t3d[s0 * 9 + e] = compose_element(a.rot + 9 * (size_t)q, sy + 9 * (e / 9), e % 9);
   }
   float2 *z = reinterpret_cast<float2 *>(dyn);
-  const unsigned short *pos = load_pos(z, per, p);
+  const unsigned short *pos = begin(z, per, p);
   const float tx = a.txy ? a.txy[2 * (size_t)q] : 0.0f, ty = a.txy ? a.txy[2 * (size_t)q + 1] : 0.0f;
-  const bool copy = fabsf(tx) < 1e-6f && fabsf(ty) < 1e-6f;
+  Shift c;
+  c.tx = tx;
+  c.ty = ty;
+  c.scale = a.scale_out;
+  c.N = N;
+  c.copy = fabsf(tx) < 1e-6f && fabsf(ty) < 1e-6f;
   auto rows = [&](const auto &at, float mean) {
-    for (Walk w(N); w.slow < count; w.next()) {
-      const int y = 2 * (j0 + w.slow), x = w.fast;
-      z[w.slow * p.ld + pad(x)] =
-          make_float2(shifted(at, N, y, x, tx, ty, copy, mean, a.scale_out),
-                      shifted(at, N, y + 1, x, tx, ty, copy, mean, a.scale_out));
+    c.mean = mean;
+    // a thread keeps a column for all of the block's rows
+    const int lines = max(1, (int)blockDim.x / N), line = lines > 1 ? threadIdx.x / N : 0;
+    if (line >= lines) return;
+    for (int x = threadIdx.x - line * N; x < N; x += blockDim.x) {
+      const Column k = column_of(c, x);
+      for (int s0 = line; s0 < count; s0 += 2 * lines) {
+        float2 v[2];
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+          const int y = 2 * (j0 + min(s0 + g * lines, count - 1));
+          v[g] = make_float2(shifted(at, c, k, y), shifted(at, c, k, y + 1));
+        }
+#pragma unroll
+        for (int g = 0; g < 2; g++)
+          if (s0 + g * lines < count) z[(s0 + g * lines) * p.ld + pad(x)] = v[g];
+      }
     }
   };
   if (has_ctf(a, q)) {
     const Image at{a.img + (size_t)q * N * N, N};
     double t = 0.0;   // the edge mean from the blocks' sums (same grid)
-    for (int i = 0; i < (int)gridDim.y; i++) t += __ldg(&a.edge[(size_t)q * gridDim.y + i]);
+    if (a.means) {
+      for (int i = threadIdx.x; i < (int)gridDim.y; i += blockDim.x)
+        t += __ldg(&a.edge[(size_t)q * gridDim.y + i]);
+      t = block_sum(t, s_red);
+    }
     rows(at, a.means ? __fdiv_rn((float)t, (float)(N * 4)) : 0.0f);
   } else {
     const Padded at = padded(a, N, q, s_red, a.means);
@@ -374,14 +464,15 @@ __global__ void __launch_bounds__(256) k_rows_shift(Args a, Plan p, int per) {
 
 // Last columns: the slice in natural order, the phase origin moved to the
 // corner (a shift by N/2, N even) by the sign (-1)^(kx+ky).
-__global__ void __launch_bounds__(256) k_cols_out(Args a, Plan p, int per) {
+__global__ void __launch_bounds__(256, 4) k_cols_out(Args a, Plan p, int per) {
   const int q = blockIdx.x, N = p.N, w2 = N / 2 + 1, c0 = blockIdx.y * per,
             count = min(per, w2 - c0);
   float2 *z = reinterpret_cast<float2 *>(dyn);
-  const unsigned short *pos = load_pos(z, per, p);
+  const unsigned short *pos = begin(z, per, p);
   float2 *spec = a.spec + (size_t)q * N * w2 + c0;
-  for (Walk w(count); w.slow < N; w.next())
-    z[w.fast * p.ld + pad(w.slow)] = spec[(size_t)w.slow * w2 + w.fast];
+  batched<8>(
+      Walk(count), N, [&](int y, int c) { return spec[(size_t)y * w2 + c]; },
+      [&](int y, int c, float2 v) { z[c * p.ld + pad(y)] = v; });
   transform<-1>(z, count, p);
   for (Walk w(count); w.slow < N; w.next()) {
     float2 v = z[w.fast * p.ld + pad(pos[w.slow])];
@@ -390,28 +481,30 @@ __global__ void __launch_bounds__(256) k_cols_out(Args a, Plan p, int per) {
   }
 }
 
-// Up to three radices whose product is N, the largest as small as it goes.
+// Up to three radices of 2 to 16 whose product is N, as few as it takes and the
+// largest as small as it goes; false where there are none.
 static bool factor(int N, std::vector<int> &out) {
-  static const int all[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16};
-  int best = 1 << 30;
-  for (int passes = 1; passes <= 3 && best == 1 << 30; passes++)
-    for (int a : all)
-      for (int b : all)
-        for (int c : all) {
-          if (passes < 3 && c != 2) break;
-          if (passes < 2 && b != 2) break;
-          const int p = a * (passes > 1 ? b : 1) * (passes > 2 ? c : 1);
-          if (p != N) continue;
-          std::vector<int> r{a};
-          if (passes > 1) r.push_back(b);
-          if (passes > 2) r.push_back(c);
-          const int worst = *std::max_element(r.begin(), r.end());
-          if (worst < best) {
-            best = worst;
-            out = r;
-          }
-        }
-  return best < (1 << 30);
+  if (N < 2 || N > 4096) return false;
+  if (N <= 16) {
+    out = {N};
+    return true;
+  }
+  int best = 17;
+  for (int a = 2; a <= 16; a++)
+    if (N % a == 0 && N / a >= 2 && std::max(a, N / a) < best) {
+      best = std::max(a, N / a);
+      out = {a, N / a};
+    }
+  if (best <= 16) return true;
+  for (int a = 2; a <= 16; a++)
+    for (int b = 2; b <= 16; b++) {
+      const int c = N / (a * b), worst = std::max(a, std::max(b, c));
+      if (N % (a * b) == 0 && c >= 2 && worst < best) {
+        best = worst;
+        out = {a, b, c};
+      }
+    }
+  return best <= 16;
 }
 
 // The plan's tables on the current device, made once per size.
@@ -471,14 +564,13 @@ static int get_plan(int N, Plan &out) {
 
 size_t lines_edge_bytes(int N, int n) { return sizeof(double) * (size_t)n * (N / 2); }
 
-// Few particles only: five short launches against ten, a call of one particle
-// with a CTF N = 192 47 against 62 us, N = 384 55 against 59; from about
-// eight on, or four of the larger sizes, the library's transforms over many
-// lines at once win (N = 192, 4: 51 against 63, 8: 70 against 63; N = 384, 2:
-// 57 against 65, 4: 87 against 70).
-bool lines_fits(int N, int n) {
+// Sizes of up to three radices; others take the library's transforms, and so do
+// many large images with a CTF, whose columns no longer come by whole 128-byte
+// lines: N = 1024, 16 511 against 516 us, 64 1882 against 1699; N = 2048, 4 600
+// against 777, 16 2260 against 2015.
+bool lines_fits(int N, int n, bool ctf) {
   std::vector<int> r;
-  return n <= (N <= 240 ? 6 : 2) && lines::factor(N, r);
+  return !(ctf && N >= 1000 && (long)n * N > 16384) && lines::factor(N, r);
 }
 
 int launch_lines(const float *d_raw, const float *const *d_src, int n, int box, int N,
@@ -504,29 +596,43 @@ int launch_lines(const float *d_raw, const float *const *d_src, int n, int box, 
   a.img = d_img;
   a.edge = d_edge;
   a.spec = d_out;
-  // lines per block: few when the call has few, so that it reaches every SM
+  // lines per block: few when the call has few, so that it reaches every SM,
+  // and no more than let four blocks share one
   const int n2 = N / 2, w2 = n2 + 1;
   const size_t line = sizeof(float2) * p.ld;
-  int per = 8;
+  int per = 16;
   while (per > 2 && ((long)n * n2 < 148L * 2 * per || line * per > 60000)) per /= 2;
   while (per > 1 && line * per + sizeof(short) * N > 220000) per /= 2;
   const size_t smem = line * per + sizeof(short) * N;
   const dim3 rows(n, (n2 + per - 1) / per), cols(n, (w2 + per - 1) / per);
-  const int threads = 256;
-  auto go = [&](void (*k)(lines::Args, lines::Plan, int), dim3 grid) {
+  // the shift's threads keep a column, or as many as it takes
+  const int turns = (N + 255) / 256, shift = N > 128 ? ((N + turns - 1) / turns + 31) / 32 * 32 : 256;
+  bool first = true;
+  auto go = [&](void (*k)(lines::Args, lines::Plan, int), dim3 grid, int threads) {
     cudaError_t e = set_max_smem((const void *)k, smem);
     if (e != cudaSuccess) return e;
     note_launch();
-    k<<<grid, threads, smem, st>>>(a, p, per);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    // each stage after the first may start while the one before it drains
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &early;
+    cfg.numAttrs = first ? 0 : 1;
+    first = false;
+    return cudaLaunchKernelEx(&cfg, k, a, p, per);
   };
   if (d_ctf) {
-    CU(go(lines::k_rows_pad, rows));
-    CU(go(lines::k_cols_flip, cols));
-    CU(go(lines::k_rows_back, rows));
+    CU(go(lines::k_rows_pad, rows, 256));
+    CU(go(lines::k_cols_flip, cols, 256));
+    CU(go(lines::k_rows_back, rows, 256));
   }
-  CU(go(lines::k_rows_shift, rows));
-  CU(go(lines::k_cols_out, cols));
+  CU(go(lines::k_rows_shift, rows, shift));
+  CU(go(lines::k_cols_out, cols, 256));
   return FR_OK;
 }
 
