@@ -172,6 +172,7 @@ struct RoundGroup {
   // units_off, nunits) with the launch's unit count
   std::vector<int> turns;
   int units = 0;
+  long patches = 0;            // of the segments (plane_patches)
   // the segments' centre copies: offset of each (job, bytes from the start of
   // the group's buffer), their total and the largest half-width
   std::vector<std::pair<int, size_t>> centres;
@@ -267,6 +268,7 @@ static void plan_plane(RoundPlan &P, RoundGroup &g) {
       g.centre_half = std::max(g.centre_half, half);
     }
     g.units = next;
+    g.patches += plane_patches(J.N, (long)J.np * J.nsym);
     g.maxN = std::max(g.maxN, J.N);
   }
   g.units_off = (P.work.size() + 15) & ~(size_t)15;
@@ -386,7 +388,7 @@ static int plan_launch_group(const RoundPlan &P, BatchScratch &bs, size_t gi, cu
   if (is_plane_group(g.tile)) {
     for (int k : g.turns) TRY(run_plane(P.hj[k], bs.plane[gi], st));
     CU(launch_plane_multi(d_jobs, (const PlaneSeg *)units, (int)g.nunits, g.units, g.max_mode,
-                          g.maxN, st));
+                          g.maxN, g.patches, st));
     if (!g.centres.empty())
       CU(launch_merge_centre(d_jobs, (int)P.hj.size(), nullptr, g.max_mode, g.centre_half, st));
     return FR_OK;
