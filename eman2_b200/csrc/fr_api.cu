@@ -1317,7 +1317,7 @@ int fr_determine_slice_agreement(fr_recon *r, const float *slices, int n, const 
   CU(launch_compose((const float *)d_rot, r->d_sym.as<float>(), n, r->nsym, r->s_t3d.as<float>(), st));
   // the blocks' sums, then the results when they go to the host
   const bool dev_out = is_device_ptr(out);
-  const size_t part = agree_scratch_bytes(N, n);
+  const size_t part = agree_scratch_bytes(N, n, r->nsym);
   TRY(r->s_out.ensure(part + sizeof(float) * 5 * n));
   float *d_out = dev_out ? out : reinterpret_cast<float *>(r->s_out.as<unsigned char>() + part);
   CU(launch_agree_rt(r->vol_data.as<float>(), r->vol_norm.as<float>(), N, (const float *)d_sl,

@@ -224,13 +224,15 @@ __device__ __forceinline__ int ref_round(float x) {
   return (int)__fadd_rn(x, 0.5f);
 }
 
-// What bounds it: L2 gathers (a pixel's value and weight, 12 bytes from two
-// scattered sectors, per symmetry copy) and the arithmetic around them.  A
+// What bounds it: gathers (a pixel's value and weight, 12 bytes from two
+// scattered sectors, per symmetry copy), from HBM for volumes beyond the L2
+// cache (72 % of its bandwidth with the whole volume at once, whence
+// agree_slabs), else from L2.  A
 // slice's rows are dealt to several blocks, so that a call of any number of
 // slices fills the device; a thread reads its pixel of the slice once and runs
 // over the copies.  Each block leaves its eight FP64 sums, and a second launch
 // adds a slice's sums in block order, so the result does not depend on timing.
-// 128 slices at N = 384, d7: 1.4 ms, against 6.6 ms with one block a slice,
+// 128 slices at N = 384, d7: 1.2 ms, against 6.6 ms with one block a slice,
 // integer and float divisions per pixel and a double square root for its
 // radius (which only enters as 3 < r < rmax: a range of integers x^2 + y^2).
 constexpr int kAgreeRows = 8;   // rows a block takes at a time, one warp each
@@ -240,7 +242,7 @@ __global__ void __launch_bounds__(256) k_agree(const float2 *__restrict__ rdata,
                                                const float *__restrict__ slices,
                                                const float *__restrict__ t3d, int nsym,
                                                const float *__restrict__ rtab, int low_end,
-                                               double *__restrict__ part) {
+                                               int slabs, double *__restrict__ part) {
   extern __shared__ float s_rot[];       // [nsym][6]
   __shared__ double s_red[8][kAgreeRows];
   const int p = blockIdx.y;
@@ -252,6 +254,8 @@ __global__ void __launch_bounds__(256) k_agree(const float2 *__restrict__ rdata,
   for (int k = threadIdx.x; k < nsym * 6; k += blockDim.x)
     s_rot[k] = t3d[((size_t)p * nsym + k / 6) * 9 + k % 6];
   __syncthreads();
+  // this block's slab of the volume: z rows [z_lo, z_hi)
+  const int z_lo = (int)((long)N * blockIdx.z / slabs), z_hi = (int)((long)N * (blockIdx.z + 1) / slabs);
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};  // dotlow dlpow dlpow2 dot vweight power power2
   int nval = 0;
   for (int row = blockIdx.x * kAgreeRows + warp; row < N; row += gridDim.x * kAgreeRows) {
@@ -270,17 +274,19 @@ __global__ void __launch_bounds__(256) k_agree(const float2 *__restrict__ rdata,
       const bool low = q > 9 && q < low_end;
       for (int s = 0; s < nsym; s++) {
         const float *M = s_rot + 6 * s;
-        float xx = __fadd_rn(__fmul_rn(rx, M[0]), __fmul_rn(ry, M[3]));
-        float yy = __fadd_rn(__fmul_rn(rx, M[1]), __fmul_rn(ry, M[4]));
-        float zz = __fadd_rn(__fmul_rn(rx, M[2]), __fmul_rn(ry, M[5]));
-        if (fabsf(xx) > 0.5f || fabsf(yy) >= 0.5f || fabsf(zz) >= 0.5f) continue;
-        xx = __fmul_rn(xx, Nf);
-        yy = __fmul_rn(yy, Nf);
-        zz = __fmul_rn(zz, Nf);
-        int x0 = ref_round(xx), y0 = ref_round(yy), z0 = ref_round(zz);
+        const float xx = __fadd_rn(__fmul_rn(rx, M[0]), __fmul_rn(ry, M[3]));
+        const float zz = __fadd_rn(__fmul_rn(rx, M[2]), __fmul_rn(ry, M[5]));
+        if (fabsf(xx) > 0.5f || fabsf(zz) >= 0.5f) continue;
+        int x0 = ref_round(__fmul_rn(xx, Nf)), z0 = ref_round(__fmul_rn(zz, Nf));
         const bool mir = x0 < 0;
-        if (mir) { x0 = -x0; y0 = -y0; z0 = -z0; }
-        const long c = (long)x0 + (long)((y0 < 0 ? N + y0 : y0) + (z0 < 0 ? N + z0 : z0) * N) * w2;
+        if (mir) z0 = -z0;
+        const int zi = z0 < 0 ? N + z0 : z0;
+        if (zi < z_lo || zi >= z_hi) continue;
+        const float yy = __fadd_rn(__fmul_rn(rx, M[1]), __fmul_rn(ry, M[4]));
+        if (fabsf(yy) >= 0.5f) continue;
+        int y0 = ref_round(__fmul_rn(yy, Nf));
+        if (mir) { x0 = -x0; y0 = -y0; }
+        const long c = (long)x0 + (long)((y0 < 0 ? N + y0 : y0) + zi * N) * w2;
         const float nv = __ldg(&norm[c]);
         float2 v = make_float2(0.f, 0.f);
         if (!(x0 >= nxf / 2 || abs(y0) > n2 || abs(z0) > n2)) {
@@ -311,19 +317,24 @@ __global__ void __launch_bounds__(256) k_agree(const float2 *__restrict__ rdata,
   if (threadIdx.x < 8) {
     double t = 0;
     for (int w = 0; w < kAgreeRows; w++) t += s_red[threadIdx.x][w];
-    part[((size_t)p * gridDim.x + blockIdx.x) * 8 + threadIdx.x] = t;
+    part[(((size_t)p * gridDim.z + blockIdx.z) * gridDim.x + blockIdx.x) * 8 + threadIdx.x] = t;
   }
 }
 
-// One thread per slice: its blocks' sums in order, and the attributes.
-__global__ void __launch_bounds__(64) k_agree_out(const double *__restrict__ part, int np,
+// One warp per slice: its blocks' sums (in an order of their own, so the result
+// does not depend on timing), and the attributes.
+__global__ void __launch_bounds__(128) k_agree_out(const double *__restrict__ part, int np,
                                                   int blocks, const float *__restrict__ wts,
                                                   float *__restrict__ out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int p = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p >= np) return;
   double t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int b = 0; b < blocks; b++)
+  for (int b = lane; b < blocks; b += 32)
     for (int k = 0; k < 8; k++) t[k] += part[((size_t)p * blocks + b) * 8 + k];
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    for (int o = 16; o; o >>= 1) t[k] += __shfl_down_sync(0xffffffffu, t[k], o);
+  if (lane) return;
   double dotlow = t[0], dlpow = t[1], dlpow2 = t[2], dot = t[3], vweight = t[4];
   const double power = t[5], power2 = t[6];
   const int nval = (int)t[7];
@@ -346,8 +357,19 @@ static int agree_blocks(int N, int np) {
   return std::max(1, std::min((N + kAgreeRows - 1) / kAgreeRows, want));
 }
 
-size_t agree_scratch_bytes(int N, int np) {
-  return sizeof(double) * 8 * (size_t)np * agree_blocks(N, np);
+// Slabs of the volume, one after another: the copies of many slices come back
+// to a cell, and find it in the L2 cache if only a part of the volume is under
+// way, for the arithmetic up to the slab's test once more per slab.  ms, one
+// slab against two (three): d7, N = 384, 128 slices 1.59, 1.18 (1.28), 32 0.44,
+// 0.35, 8 0.16, 0.18; N = 256, 128 0.42, 0.49; N = 640, 64 3.63, 3.11 (2.84);
+// c1, N = 384, 600 0.66, 0.74.
+static int agree_slabs(int N, int np, int nsym) {
+  const double mb = 6e-6 * N * N * (double)N;
+  return nsym == 1 || mb < 190 || (long)np * nsym < N ? 1 : mb < 750 ? 2 : 3;
+}
+
+size_t agree_scratch_bytes(int N, int np, int nsym) {
+  return sizeof(double) * 8 * (size_t)np * agree_blocks(N, np) * agree_slabs(N, np, nsym);
 }
 
 cudaError_t launch_agree_rt(const float *d_data, const float *d_norm, int N, const float *d_slices,
@@ -362,17 +384,18 @@ cudaError_t launch_agree_rt(const float *d_data, const float *d_norm, int N, con
   int low_end = rmax == rmax ? (int)std::min(2.0e9, (double)rmax * rmax + 1) : 0;
   while (low_end > 0 && (float)std::sqrt((double)(low_end - 1)) >= rmax) low_end--;
   const int per = 65535;   // grid.y
-  const int blocks = agree_blocks(N, np);
+  const int blocks = agree_blocks(N, np), slabs = agree_slabs(N, np, nsym);
   const size_t smem = sizeof(float) * 6 * nsym;
   for (int p0 = 0; p0 < np; p0 += per) {
     const int n = std::min(per, np - p0);
     note_launch();
-    k_agree<<<dim3(blocks, n), 256, smem, st>>>(
+    k_agree<<<dim3(blocks, n, slabs), 256, smem, st>>>(
         reinterpret_cast<const float2 *>(d_data), d_norm, N, d_slices + (size_t)p0 * N * (N + 2),
-        d_t3d + (size_t)p0 * nsym * 9, nsym, d_rtab, low_end, d_part + (size_t)p0 * blocks * 8);
+        d_t3d + (size_t)p0 * nsym * 9, nsym, d_rtab, low_end, slabs,
+        d_part + (size_t)p0 * blocks * slabs * 8);
   }
   note_launch();
-  k_agree_out<<<(np + 63) / 64, 64, 0, st>>>(d_part, np, blocks, d_w, d_out);
+  k_agree_out<<<(np + 3) / 4, 128, 0, st>>>(d_part, np, blocks * slabs, d_w, d_out);
   return cudaGetLastError();
 }
 

@@ -268,7 +268,7 @@ cudaError_t launch_finish_out(const float *d_real_padded, int N, float scale, fl
 cudaError_t launch_seed(const float *d_seed, float w, int N, float *d_data, float *d_norm,
                         cudaStream_t st);
 // d_part: agree_scratch_bytes of workspace.
-size_t agree_scratch_bytes(int N, int np);
+size_t agree_scratch_bytes(int N, int np, int nsym);
 cudaError_t launch_agree_rt(const float *d_data, const float *d_norm, int N, const float *d_slices,
                             const float *d_t3d, int np, int nsym, const float *d_w, float apix,
                             const float *d_rtab, double *d_part, float *d_out, cudaStream_t st);

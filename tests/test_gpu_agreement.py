@@ -31,3 +31,23 @@ def test_agreement_sizes(gpu, N, n, sym, apix):
     for i in range(n):
         np.testing.assert_allclose(got[i], o.compare(sl[i], rt[i], float(w[i]), sym, apix),
                                    rtol=2e-5, atol=2e-6)
+
+
+@pytest.mark.parametrize("N,n", [(318, 23), (506, 37)])
+def test_agreement_slabs(gpu, N, n):
+    """Volumes beyond the L2 cache are taken in two or three slabs when many
+    slices are compared at once, whole when few are: the same FP64 sums in
+    another order, so the attributes agree to the rounding to float."""
+    from eman2_b200 import Reconstructors
+    from eman2_b200.synth import quaternion_blocks, random_quaternions
+    rng = np.random.default_rng(N)
+    sl = rng.normal(size=(n, N, N + 2)).astype(np.float32)
+    rt = quaternion_blocks(random_quaternions(n, rng))
+    w = rng.uniform(0.2, 1.0, n).astype(np.float32)
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "d7", "mode": "gauss_2"})
+    r.setup()
+    r.insert_slices(sl, rt, w)
+    got = r.slice_agreement(sl, rt, w)
+    for i in range(0, n, 7):
+        np.testing.assert_allclose(got[i], r.slice_agreement(sl[i:i + 1], rt[i:i + 1], w[i:i + 1])[0],
+                                   rtol=3e-7, atol=1e-7)
