@@ -138,10 +138,10 @@ def load_peaks():
 
 
 def load_traffic(workload: str, batch: int):
-    """DRAM bytes (read + write) of one insertion launch of this workload and
-    batch, from the committed ncu capture of the same bench command; None
+    """DRAM bytes (read + write) of one insertion call of this workload and
+    batch (all of its launches), from the committed ncu capture of the same bench command; None
     when no capture of that size exists."""
-    path = os.path.join(ROOT, "profiles", "k_column3_dram.json")
+    path = os.path.join(ROOT, "profiles", "insertion_dram.json")
     try:
         with open(path) as f:
             e = json.load(f)[workload]
@@ -798,15 +798,15 @@ def run_target(dev, steps: int = 3, plain_n: int = 64):
     taps = nsym_of(wl["sym"]) * pixels_per_slice(N) * 8 * 2048 / (gms / 1e3)
     upd = update_peaks()
     out = {"workload": wl["desc"], "batched": {"value": batched, "unit": "particle-slices/s",
-                                               "particles_per_call": 2048, "kernel": "k_pixel",
+                                               "particles_per_call": 2048, "kernel": "k_plane",
                                                "avg_launch_ms": gms},
            "plain": {"value": plain, "unit": "particle-slices/s", "sample": plain_n,
                      "kernel": "k_scatter"},
            "batched_vs_plain": batched / plain}
     if upd is not None:
-        out["update_roofline"] = {"bound": "shared-memory FP32 atomics (3 per tap)",
-                                  "achieved": taps, "peak": upd["smem_atom"], "unit": "taps/s",
-                                  "frac": taps / upd["smem_atom"]}
+        out["update_roofline"] = {"bound": "shared-memory float4 read-modify-write",
+                                  "achieved": taps, "peak": upd["smem_rmw"], "unit": "taps/s",
+                                  "frac": taps / upd["smem_rmw"]}
     # the HBM roofline of the same launch, as the main line's (algorithmic
     # bytes over the launch time) with its committed DRAM traffic
     peak, peak_kind = load_peaks()
@@ -985,7 +985,8 @@ def main():
     alg_bytes = args.batch * (8 * (N // 2 + 1) * N + 64) + 24 * V
     if st["gather_launches"] > 0:
         # the library's default: k_plane, and k_pixel for the narrow windows of large volumes
-        plane = wl["mode"] == "gauss_5" or (wl["mode"] != "nearest_neighbor" and N <= 352)
+        most = {"gauss_5": N, "gauss_2": 432, "trilinear": 352}.get(wl["mode"], 0)
+        plane = N <= most
         tile = args.tile if args.tile not in (-1, 5, 6) else (5 if plane else 6)
         kname = {6: "k_pixel", 5: "k_plane", 4: "k_column"}.get(tile, "k_gather") + \
             " (gather schedule)"
@@ -1018,8 +1019,9 @@ def main():
     }
     if upd is not None:
         # the binding roof: the rate of the accumulator update the kernel
-        # uses (the column kernel: one shared float4 read-modify-write per
-        # tap; the pixel kernel: three shared FP32 atomics; the scatter:
+        # uses (the column kernels: one shared read-modify-write per tap,
+        # which gauss_5's plane columns mostly save by summing in registers;
+        # the pixel kernel: three shared FP32 atomics; the scatter:
         # three L2 reductions)
         key = ("l2_red" if st["gather_launches"] == 0 else
                "smem_atom" if kname.startswith("k_pixel") else "smem_rmw")
