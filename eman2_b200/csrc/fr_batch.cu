@@ -250,12 +250,17 @@ static void plan_units(RoundPlan &P, RoundGroup &g, bool edge) {
 static void plan_plane(RoundPlan &P, RoundGroup &g) {
   std::vector<PlaneSeg> segs;
   g.max_mode = g.tile - kPlaneGroup;
+  long slices = 0;   // of the shared launch: each takes the parts that fill the device together
+  for (size_t k = 0; k < P.hj.size(); k++) {
+    const long n = (long)P.hj[k].np * P.hj[k].nsym;
+    if (P.jt[k] == g.tile && !plane_partial(P.hj[k].N, n)) slices += n;
+  }
   for (size_t k = 0; k < P.hj.size(); k++) {
     if (P.jt[k] != g.tile) continue;
     const InsertJob &J = P.hj[k];
     PlaneSeg q;
     int next = -1;
-    if (!plane_partial(J.N, (long)J.np * J.nsym)) next = plane_seg(J, (int)k, g.units, q);
+    if (!plane_partial(J.N, (long)J.np * J.nsym)) next = plane_seg(J, (int)k, g.units, slices, q);
     if (next < 0) {
       g.turns.push_back((int)k);
       continue;

@@ -147,12 +147,14 @@ cudaError_t launch_plane(const InsertJob &j, cudaStream_t st);
 // The same with caller-supplied exp table and Gaussian factor.
 cudaError_t launch_plane_tables(const InsertJob &j, const float *table, float h, cudaStream_t st);
 // Several jobs of one mode in one launch: segment i's job has `parts` units
-// per slice, numbered from `first` on.  plane_seg fills a segment and returns
-// the next first unit (-1: more units than an int holds).
+// per slice, numbered from `first` on.  plane_seg fills a segment of a launch
+// of so many slices in all (which their parts fill together: 64 jobs of one
+// empty particle each took 3.5 us apiece cut as if alone) and returns the next
+// first unit (-1: more units than an int holds).
 struct PlaneSeg {
   int job, first, parts;
 };
-int plane_seg(const InsertJob &j, int job, int first, PlaneSeg &out);
+int plane_seg(const InsertJob &j, int job, int first, long slices, PlaneSeg &out);
 cudaError_t launch_plane_multi(const InsertJob *d_jobs, const PlaneSeg *d_segs, int nsegs,
                                int units, int mode, int maxN, long patches, cudaStream_t st);
 // Patches of columns of so many slices (about three quarters of a bounding box's).

@@ -806,12 +806,11 @@ static int plane_parts(int N, int mode, long slices) {
   return (int)std::min(most, std::max(fine, fill));
 }
 
-int plane_seg(const InsertJob &j, int job, int first, PlaneSeg &out) {
-  const long slices = (long)j.np * j.nsym;
+int plane_seg(const InsertJob &j, int job, int first, long slices, PlaneSeg &out) {
   out.job = job;
   out.first = first;
   out.parts = plane_parts(j.N, j.mode, slices);
-  const long end = first + slices * out.parts;
+  const long end = first + (long)j.np * j.nsym * out.parts;
   return end > INT_MAX ? -1 : (int)end;
 }
 
