@@ -197,9 +197,9 @@ cudaError_t launch_pixel(const InsertJob *d_jobs, const int4 *d_work, int nwork,
 // two-tap windows' runs are short, so far beyond the L2 cache the plane-column
 // kernel waits for memory on every run, while the tile kernel adds to a tile
 // many times before it flushes it.  gauss_2, d7, plane against tile, us a
-// particle: N = 288 21.6, 26.2; N = 384 39.7, 43.7 (37 particles 43.6, 47.0);
-// N = 480 66, 68 (32 particles 86, 75); N = 640 121, 121.  trilinear, N = 384
-// 43.1, 42.4.
+// particle: N = 288 21.6, 26.2; N = 384 35.4, 42.8 (37 particles 43.6, 47.0);
+// N = 480 62, 68 (32 particles 81, 75); N = 640 117, 121 (32 160, 137).
+// trilinear, N = 384 42.2, 42.4.
 inline int effective_tile(int tile, int mode, int N) {
   if (tile != kPlaneTile && tile != kPixelTile) return tile;
   const int most = mode == 5 ? INT_MAX : (mode == 2 ? 432 : 352);

@@ -17,24 +17,24 @@
 // beyond it (gauss_2, d7, N = 384: 47.4 us a particle with two a cell, 37.0
 // with the value's alone, 34.4 with none), by the request rather than by the
 // byte.  So a large call's partial volume holds a cell's value and weight
-// together, one 16-byte reduction (39.4), and a run's cells are addressed by a
-// stride.  Walking eight neighbouring columns in step, which puts their
+// together, one 16-byte reduction (39.4, and 35.4 with the patches drawn), and
+// a run's cells are addressed by a stride.  Walking eight neighbouring columns in step, which puts their
 // reductions into one line, took more instructions than it saved (45.0).
 //
-// What bounds it: issue slots (76 % of cycles issue at gauss_5, 75 % at
-// gauss_2 while the volume fits L2), at 69 % of lanes busy: the windows of a
-// warp's columns hold unequal pixel counts.  A gauss_5 tap takes 36 thread
+// What bounds it: issue slots (68 % of cycles issue at gauss_5, whose registers
+// leave 16 warps an SM, 78 % at gauss_2), at 69 % of lanes busy: the windows of
+// a warp's columns hold unequal pixel counts.  A gauss_5 tap takes 36 thread
 // instructions, 64 in the tile columns: a pixel's coordinates and window serve
 // six taps, the weights go through packed operations, and a cell leaves the
 // registers once.
 // Measured on one B200, insertion alone (the kernels it took over from in
-// parentheses): gauss_5, d7, N = 384, 64 particles 19.5 ms (46.8, tile columns
-// with shared read-modify-writes), one particle 0.43 ms (1.32, an atomic per
-// tap); gauss_2, c1, N = 192, 2048 particles 1.46 ms (2.12, tiles with shared
+// parentheses): gauss_5, d7, N = 384, 64 particles 17.9 ms (46.8, tile columns
+// with shared read-modify-writes), one particle 0.35 ms (1.32, an atomic per
+// tap); gauss_2, c1, N = 192, 2048 particles 1.41 ms (2.12, tiles with shared
 // atomics).  Blocks an SM: gauss_5 without spills (two of eight warps, 128
-// registers) against three at 80, 20.1 against 21.6 ms; five or four of four
-// warps 20.8 and 20.3.  The two-tap windows at three blocks 1.52 ms, two 1.70,
-// four 1.60, five 1.71 (spills).
+// registers) against three at 80, 20.1 against 21.6 ms with the patches dealt
+// out; five or four of four warps 20.8 and 20.3.  The two-tap windows at three
+// blocks 1.52 ms, two 1.70, four 1.60, five 1.71 (spills).
 //
 // Tap selection and weights are the reference's bit for bit (window start,
 // exp-table index, radius); a cell's taps of one slice are summed before they
