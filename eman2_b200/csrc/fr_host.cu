@@ -6,6 +6,10 @@
 // 1.3 ms.  Here several threads each take pieces of the result through two
 // pinned buffers of their own: while one piece crosses the bus, the one before
 // is copied out, and the page faults are spread over the threads.
+//
+// The threads queue their copies on a stream of the pool, which waits for an
+// event that the calling thread records: the caller's stream handle may name
+// another stream in another thread (cudaStreamPerThread does).
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -24,11 +28,37 @@ constexpr int kThreads = 8;
 constexpr size_t kLeast = 4u << 20;   // smaller results: a plain copy
 
 // The pinned buffers: two pieces per thread, 32 MiB in all, one set for the
-// process.  A copy that finds them taken by another thread's goes the plain
-// way; they are freed with the last handle.
+// process, with the copies' stream and event on the device of the last copy.
+// A copy that finds them taken by another thread's goes the plain way; they
+// are freed with the last handle.
 struct Pool {
   std::mutex use;
   unsigned char *p = nullptr;
+  int dev = -1;
+  cudaStream_t st = nullptr;
+  cudaEvent_t ready = nullptr;
+
+  void drop_stream() {
+    if (st) cudaStreamDestroy(st);
+    if (ready) cudaEventDestroy(ready);
+    st = nullptr;
+    ready = nullptr;
+    dev = -1;
+  }
+  // Lets the pool's stream go on from where `user` is now.
+  bool follow(cudaStream_t user, int device) {
+    if (dev != device) {
+      drop_stream();
+      if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
+          cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) != cudaSuccess) {
+        drop_stream();
+        return false;
+      }
+      dev = device;
+    }
+    return cudaEventRecord(ready, user) == cudaSuccess &&
+           cudaStreamWaitEvent(st, ready, 0) == cudaSuccess;
+  }
 } g_pool;
 std::atomic<int> g_handles{0};
 
@@ -69,6 +99,7 @@ void host_pool_leave() {
   if (g_handles > 0 || !g_pool.p) return;
   cudaFreeHost(g_pool.p);
   g_pool.p = nullptr;
+  g_pool.drop_stream();
 }
 
 // Copies device memory to pageable host memory, after the work queued on st,
@@ -85,13 +116,17 @@ bool copy_to_pageable(void *dst, const void *dsrc, size_t bytes, cudaStream_t st
   }
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (!g_pool.follow(st, dev)) {
+    cudaGetLastError();
+    return false;
+  }
   const int threads = (int)std::min<size_t>(
       std::min<unsigned>(kThreads, std::max(1u, std::thread::hardware_concurrency())),
       (bytes + kPiece - 1) / kPiece);
   std::atomic<bool> ok{true};
   auto work = [&](int t) {
     if (!one_thread(g_pool.p + 2 * t * kPiece, static_cast<unsigned char *>(dst),
-                    static_cast<const unsigned char *>(dsrc), bytes, t, threads, dev, st))
+                    static_cast<const unsigned char *>(dsrc), bytes, t, threads, dev, g_pool.st))
       ok = false;
   };
   std::vector<std::thread> others;

@@ -57,3 +57,24 @@ def test_finish_weights_only_when_asked(gpu, tmp_path):
         assert np.array_equal(r.finish(True).numpy(), plain)
     assert np.array_equal(out.numpy(), np.load(tmp_path / "n.npy"))
     assert out.numpy().shape == (48, 48, 25)
+
+
+def _per_thread_stream(r):
+    """The handle on the per-thread default stream (cudaStreamPerThread)."""
+    from eman2_b200 import _lib
+    _lib.check(_lib.load().fr_set_stream(r.handle, 2))
+
+
+@pytest.mark.parametrize("N", [64, 128, 190])
+def test_finish_on_the_per_thread_stream(gpu, N):
+    """A map copied out behind work still queued on the per-thread stream,
+    whose handle names another stream in every thread, is the one that an
+    ordinary stream gives."""
+    import torch
+    r, d, w = _seeded(N, N)
+    want = r.finish(True).numpy()
+    r, _, _ = _seeded(N, N)
+    _per_thread_stream(r)
+    with torch.cuda.stream(torch.cuda.ExternalStream(2)):
+        torch.cuda._sleep(50_000_000)
+    assert np.array_equal(r.finish(True).numpy(), want)
