@@ -380,7 +380,7 @@ int check_state(fr_recon *r) {
 }
 
 int stream_enter(fr_recon *r, cudaStream_t st) {
-  if (r->last && r->last != st) CU(cudaStreamWaitEvent(st, r->done->ev, 0));
+  if (r->last && !same_stream(r->last, st)) CU(cudaStreamWaitEvent(st, r->done->ev, 0));
   return FR_OK;
 }
 

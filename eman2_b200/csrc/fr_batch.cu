@@ -552,7 +552,7 @@ static int batch_insert(std::vector<fr_recon *> &jobs, BatchScratch &bs, int til
   // Work goes to `st` after each handle's and the scratch's earlier work on
   // other streams; the call returns once everything is enqueued.
   if (!bs.done) CU(cudaEventCreateWithFlags(&bs.done, cudaEventDisableTiming));
-  if (bs.last && bs.last != st) CU(cudaStreamWaitEvent(st, bs.done, 0));
+  if (bs.last && !same_stream(bs.last, st)) CU(cudaStreamWaitEvent(st, bs.done, 0));
   for (int j = 0; j < nj; j++) TRY(stream_enter(jobs[j], st));
   // Rounds of at most `chunk` particles per job, so scratch stays bounded.
   const int chunk = kBatchChunk;

@@ -38,6 +38,12 @@ int fail(int code, const char *fmt, ...);
     if (rc_ != FR_OK) return rc_; \
   } while (0)
 
+// Whether work queued on `now` follows work queued earlier on `before` without
+// an event: the same handle, unless it names a stream per host thread.
+inline bool same_stream(cudaStream_t before, cudaStream_t now) {
+  return before == now && now != cudaStreamPerThread;
+}
+
 struct DevBuf {
   void *p = nullptr;
   size_t cap = 0;

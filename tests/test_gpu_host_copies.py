@@ -78,3 +78,32 @@ def test_finish_on_the_per_thread_stream(gpu, N):
     with torch.cuda.stream(torch.cuda.ExternalStream(2)):
         torch.cuda._sleep(50_000_000)
     assert np.array_equal(r.finish(True).numpy(), want)
+
+
+def test_per_thread_stream_from_two_threads(gpu):
+    """Insertions that one thread queued on its per-thread stream are in the map
+    that another thread takes from its own."""
+    import torch
+    from eman2_b200 import Reconstructors
+    N, n = 48, 20
+    rng = np.random.default_rng(3)
+    sl = rng.normal(size=(n, N, N + 2)).astype(np.float32)
+    rots = np.stack([np.linalg.qr(rng.normal(size=(3, 3)))[0] for _ in range(n)]).astype(np.float32)
+
+    def inserted(per_thread):
+        r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
+        r.setup()
+        if per_thread:
+            _per_thread_stream(r)
+            with torch.cuda.stream(torch.cuda.ExternalStream(2)):
+                torch.cuda._sleep(50_000_000)
+        r.insert_slices(sl, rots, np.ones(n, np.float32))
+        return r
+
+    want = inserted(False).finish(True).numpy()
+    made = []
+    t = threading.Thread(target=lambda: made.append(inserted(True)))
+    t.start()
+    t.join()
+    got = made[0].finish(True).numpy()
+    assert np.abs(got - want).max() < 1e-5 * np.abs(want).max()
