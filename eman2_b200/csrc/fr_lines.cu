@@ -247,7 +247,7 @@ __device__ __forceinline__ Column column_of(const Shift &c, int x) {
   const int h = c.N / 2;
   const float x2 = __fadd_rn(__fadd_rn((float)(x - h), c.tx), (float)h);
   Column k;
-  k.in = x2 >= 0 && x2 < c.N;
+  k.in = !(x2 < 0 || x2 >= c.N);   // a NaN shift is not outside: its slice is NaN
   k.ix = c.copy ? x : k.in ? (int)x2 : 0;
   k.jx = k.ix == c.N - 1 ? k.ix : k.ix + 1;
   k.t = __fsub_rn(x2, (float)k.ix);
@@ -260,7 +260,7 @@ __device__ __forceinline__ float shifted(const F &at, const Shift &c, const Colu
   const int h = c.N / 2;
   const float y2 = __fadd_rn(__fadd_rn((float)(y - h), c.ty), (float)h);
   // outside: 0, after loads that wait for no test
-  const bool in = k.in && y2 >= 0 && y2 < c.N;
+  const bool in = k.in && !(y2 < 0 || y2 >= c.N);
   const int iy = in ? (int)y2 : 0, jy = iy == c.N - 1 ? iy : iy + 1;
   const float u = __fsub_rn(y2, (float)iy), omu = __fsub_rn(1.0f, u);
   const float a = at(iy, k.ix), b = at(iy, k.jx), d = at(jy, k.ix), e = at(jy, k.jx);

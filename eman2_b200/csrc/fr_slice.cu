@@ -352,13 +352,13 @@ __device__ __forceinline__ void translate(float2 *z, const Shape &s, float tx, f
   const int lines = blockDim.x / N, line = threadIdx.x / N, x = threadIdx.x - line * N;
   const bool on = line < lines;
   const float x2 = __fadd_rn(__fadd_rn((float)(x - h), tx), (float)h);
-  const bool okx = x2 >= 0 && x2 < N;
+  const bool okx = !(x2 < 0 || x2 >= N);   // a NaN shift is not outside: its slice is NaN
   const int ix = okx ? (int)x2 : 0, dx = ix == N - 1 ? 0 : 2;   // to the next column, in floats
   const float t = __fsub_rn(x2, (float)ix), omt = __fsub_rn(1.0f, t);
   const float *col = reinterpret_cast<const float *>(z) + 2 * ix;
   auto value = [&](int y) {
     const float y2 = __fadd_rn(__fadd_rn((float)(y - h), ty), (float)h);
-    if (!(okx && y2 >= 0 && y2 < N)) return 0.0f;
+    if (!okx || y2 < 0 || y2 >= N) return 0.0f;
     const int iy = (int)y2, jy = iy == N - 1 ? iy : iy + 1;
     const float u = __fsub_rn(y2, (float)iy), omu = __fsub_rn(1.0f, u);
     const float *p = col + 2 * (iy >> 1) * s.ld + (iy & 1), *q = col + 2 * (jy >> 1) * s.ld + (jy & 1);

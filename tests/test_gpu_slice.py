@@ -130,3 +130,24 @@ def test_slices_over_images(gpu, N, n, shift):
     got = buf[:n * N * (N + 2)].cpu().numpy().reshape(n, N, N + 2)
     for i in range(n):
         assert oracle.rel_l2(got[i], want[i]) < RTOL, i
+
+
+@pytest.mark.parametrize("N,n", [(32, 64), (32, 3), (170, 30), (242, 2), (52, 60)])
+@pytest.mark.parametrize("axis", [(0,), (1,), (0, 1)])
+def test_nan_shift_gives_a_nan_slice(gpu, N, n, axis):
+    """A shift that is not a number makes its slice so, in each preparation (one
+    launch, with the radix 17 too, and lines), and leaves the others alone."""
+    from eman2_b200 import Reconstructors, _lib
+    rng = np.random.default_rng(N)
+    img = rng.normal(size=(n, N, N)).astype(np.float32)
+    inv = rng.uniform(-2, 2, (n, 2)).astype(np.float32)
+    inv[1, list(axis)] = np.nan
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
+    r.setup()
+    out = np.empty((n, N, N + 2), np.float32)
+    _lib.check(_lib.load().fr_preprocess_slices(r.handle, _lib.ptr(img), n, _lib.ptr(inv),
+                                                _lib.ptr(out)))
+    assert np.isnan(out[1]).all()
+    for i in (0, n - 1):
+        want = oracle.preprocess_slice(img[i], float(inv[i, 0]), float(inv[i, 1]))
+        assert i == 1 or oracle.rel_l2(out[i], want) < RTOL, i
