@@ -209,11 +209,14 @@ struct Padded {
     return __fsub_rn(__ldg(&src[(size_t)y * box + x]), mean);
   }
 };
+// The image after the phase flip.  A stage runs beside the one before it until
+// its grid dependency is resolved, so what that one writes (these images, their
+// edge sums, the half spectra) is never read through the non-coherent path.
 struct Image {
   const float *img;
   int N;
   __device__ __forceinline__ float operator()(int y, int x) const {
-    return __ldg(&img[(size_t)y * N + x]);
+    return img[(size_t)y * N + x];
   }
 };
 
@@ -449,7 +452,7 @@ __global__ void __launch_bounds__(256, 4) k_rows_shift(Args a, Plan p, int per) 
     double t = 0.0;   // the edge mean from the blocks' sums (same grid)
     if (a.means) {
       for (int i = threadIdx.x; i < (int)gridDim.y; i += blockDim.x)
-        t += __ldg(&a.edge[(size_t)q * gridDim.y + i]);
+        t += a.edge[(size_t)q * gridDim.y + i];
       t = block_sum(t, s_red);
     }
     rows(at, a.means ? __fdiv_rn((float)t, (float)(N * 4)) : 0.0f);

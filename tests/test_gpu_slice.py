@@ -151,3 +151,31 @@ def test_nan_shift_gives_a_nan_slice(gpu, N, n, axis):
     for i in (0, n - 1):
         want = oracle.preprocess_slice(img[i], float(inv[i, 0]), float(inv[i, 1]))
         assert i == 1 or oracle.rel_l2(out[i], want) < RTOL, i
+
+
+@pytest.mark.parametrize("box,N,n", [(200, 300, 57), (290, 432, 49), (330, 500, 3), (512, 768, 1)])
+def test_lines_of_many_or_large_images(gpu, box, N, n):
+    """The line preparation where several blocks' stages overlap: many particles
+    a call and sizes beyond 384, each stage reading what the one before it wrote.
+    Without astigmatism, so that no sign hangs on the last place of an angle."""
+    from eman2_b200 import Reconstructors
+    from eman2_b200.particles import particle_meta
+    from eman2_b200.synth import quaternion_blocks, random_quaternions
+    rng = np.random.default_rng(N)
+    img = (rng.normal(size=(n, box, box)) + 3.0).astype(np.float32)
+    rots = quaternion_blocks(random_quaternions(n, rng))
+    shifts = rng.uniform(-5, 5, (n, 2)).astype(np.float32)
+    df = rng.uniform(0.8, 2.5, n).astype(np.float32)
+    df[1::4] = 0.0
+    w = rng.uniform(0.5, 1.0, n).astype(np.float32)
+    ctf = {"voltage": 300.0, "cs": 2.7}
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "nearest_neighbor"})
+    r.setup()
+    r.insert_particles(img, particle_meta(rots, shifts, w, ctf=ctf, defocus=df))
+    d, nm = r.get_accumulators()
+    sl = np.stack([oracle.particle_to_slice(img[i], N, shifts[i], dict(ctf, defocus=float(df[i])))
+                   for i in range(n)])
+    o = oracle.OracleVolume(N, "fp32acc64")
+    o.insert(sl, rots, w, "nearest_neighbor", "c1")
+    assert oracle.rel_l2(nm, o.norm) < 2e-6
+    assert oracle.rel_l2(d, o.data) < RTOL
