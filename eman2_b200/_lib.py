@@ -86,6 +86,8 @@ SIGNATURES = {
     "fr_autotune": ([ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _I, _F],
                     ctypes.c_int),
     "fr_set_tile": ([ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int], ctypes.c_int),
+    "fr_insertion_kernel": ([ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int],
+                            ctypes.c_int),
     "fr_update_peaks": ([_P, _P, _P], ctypes.c_int),
     "fr_set_wiener": ([_P, ctypes.c_int], ctypes.c_int),
     "fr_set_reference": ([_P, _P, ctypes.c_int], ctypes.c_int),

@@ -88,6 +88,12 @@ def set_tile(N: int, mode: str, nsym: int, tile: int):
     _lib.check(_lib.load().fr_set_tile(int(N), _lib.MODE_IDS[mode], int(nsym), int(tile)))
 
 
+def insertion_kernel(N: int, mode: str, nsym: int, n: int, schedule: str = "auto") -> int:
+    """The id (as TILE_NAMES) of the kernel that n slices of a cubic job take."""
+    return _lib.load().fr_insertion_kernel(int(N), _lib.MODE_IDS[mode], int(nsym), int(n),
+                                           _lib.SCHED[schedule])
+
+
 class InsertGraph:
     """A batched insertion round of fixed shapes captured once as a CUDA graph
     (fr_graph_create): every replay inserts counts[j] particles of box

@@ -473,7 +473,7 @@ int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st) {
   InsertJob j = j0;
   int half;
   const size_t cbytes = plane_centre(N, slices, half, j.copies);
-  if (cbytes && !plane_small(j.mode, N, slices) && b.centre.cap >= cbytes) {
+  if (cbytes && b.centre.cap >= cbytes) {
     j.cdata = b.centre.as<float>();
     j.centre = half;
   }
@@ -493,6 +493,36 @@ int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st) {
   return FR_OK;
 }
 
+Route insertion_route(int mode, int N, int NZ, int nsym, int np, int schedule, bool plain,
+                      int tile) {
+  const int tuned = tuned_tile(N, mode, nsym);
+  // the iterative inserter and non-cubic volumes: scatter only
+  int sched = (mode == FR_MODE_ITER || NZ != N) ? FR_SCHED_SCATTER : schedule;
+  if (sched == FR_SCHED_AUTO) {
+    // Few slices: the per-tile culling and the volume read/write of the gather
+    // pass are not amortised, so atomics win; a measured choice overrides.
+    const long slices = (long)np * nsym;
+    if (slices < 64) sched = FR_SCHED_SCATTER;
+    else if (tuned == kScatterTile) sched = FR_SCHED_SCATTER;
+    else if (tuned >= 0) sched = FR_SCHED_GATHER;
+    else sched = (slices >= 256 && mode != FR_MODE_NEAREST) ? FR_SCHED_GATHER : FR_SCHED_SCATTER;
+  }
+  Route q;
+  q.gather = sched != FR_SCHED_SCATTER && plain;
+  const int pin = tile >= 0 ? tile : tuned;
+  q.kernel = q.gather ? effective_tile(pin >= 0 ? pin : default_tile(mode, N, nsym, np), mode)
+                      : kScatterTile;
+  // the plane-column kernel also takes the calls the scatter schedule names,
+  // unless they need its per-pixel weights or its z size; a few small slices
+  // that nobody asked it for go the other way
+  const bool columns = plane_mode(mode) && NZ == N && plain;
+  if (columns && q.kernel == kScatterTile) q.kernel = kPlaneTile;
+  if (q.kernel == kPlaneTile && !(q.gather && pin == kPlaneTile) &&
+      plane_small(mode, N, (long)np * nsym))
+    q.kernel = kScatterTile;
+  return q;
+}
+
 // Inserts np device slices (t3d already composed, weights per particle).
 int insert_device(fr_recon *r, const float2 *d_slices, const float *d_t3d, const float *d_pw,
                          int np, int schedule, const float *d_ssnr, int nssnr) {
@@ -504,33 +534,17 @@ int insert_device(fr_recon *r, const float2 *d_slices, const float *d_t3d, const
     j.nssnr = nssnr;
     j.sscale = (float)(2.0 * (nssnr - 1) / (float)r->N);
   }
-  const int tuned = tuned_tile(r->N, r->mode, r->nsym);
-  // the iterative inserter and non-cubic volumes: scatter only
-  int sched = (r->mode == FR_MODE_ITER || r->NZ != r->N) ? FR_SCHED_SCATTER : schedule;
-  if (sched == FR_SCHED_AUTO) {
-    // Few slices: the per-tile culling and the volume read/write of the gather
-    // pass are not amortised, so atomics win; a measured choice overrides.
-    const long slices = (long)np * r->nsym;
-    if (slices < 64) sched = FR_SCHED_SCATTER;
-    else if (tuned == -2) sched = FR_SCHED_SCATTER;
-    else if (tuned >= 0) sched = FR_SCHED_GATHER;
-    else sched = (slices >= 256 && r->mode != FR_MODE_NEAREST) ? FR_SCHED_GATHER : FR_SCHED_SCATTER;
-  }
+  const Route route =
+      insertion_route(r->mode, r->N, r->NZ, r->nsym, np, schedule, !d_ssnr, r->tile);
+  const bool gather = route.gather, plane = route.kernel == kPlaneTile;
+  const int tile = route.kernel;
   const bool prof = g_profile.load() != 0;
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   if (prof)
     for (auto &e : ev) CU(cudaEventCreate(&e));
   g_ins_launches++;
   g_slices += (long long)np * r->nsym;
-  // the tile of a gather call; the plane-column kernel also takes the calls
-  // the scatter schedule names, unless they need its per-pixel weights or its
-  // z size
-  int tile = r->tile >= 0 ? r->tile : (tuned >= 0 ? tuned : default_tile(r->mode, r->N, r->nsym, np));
-  tile = effective_tile(tile, r->mode, r->N);
-  const bool gather = sched != FR_SCHED_SCATTER && !d_ssnr;
-  const bool plane = plane_mode(r->mode) && r->NZ == r->N && !d_ssnr &&
-                     (!gather || tile == kPlaneTile);
-  if (plane || !gather) {
+  if (plane || tile == kScatterTile) {
     if (prof) CU(cudaEventRecord(ev[0], st));
     if (plane) {
       r->plane.ensure(r->N, (long)np * r->nsym, st);
@@ -838,6 +852,10 @@ int fr_sym_ops(const char *sym, float *out, int cap) {
     memcpy(out, v.data(), sizeof(float) * 9 * n);
   }
   return n;
+}
+
+int fr_insertion_kernel(int N, int mode, int nsym, int n, int schedule) {
+  return insertion_route(mode, N, N, nsym, n, schedule, true, -1).kernel;
 }
 
 int fr_create(const fr_params *p, fr_recon **out) {

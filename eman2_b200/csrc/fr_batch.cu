@@ -27,7 +27,6 @@ namespace fr {
 // Choices per (N, mode, nsym): >= 0 gather with that tile, -2 scatter.
 static std::mutex g_tune_mu;
 static std::map<std::tuple<int, int, int>, int> g_tuned;
-constexpr int kTunedScatter = -2;
 // Particles per job per round of a batched insertion (bounds the scratch).
 constexpr int kBatchChunk = 4096;
 
@@ -37,9 +36,27 @@ int tuned_tile(int N, int mode, int nsym) {
   return it == g_tuned.end() ? -1 : it->second;
 }
 
+// The two-tap windows' runs are short, so far beyond the L2 cache the
+// plane-column kernel waits for memory on every run, while the tile kernel adds
+// to a tile many times before it flushes it: once enough slices share the tiles
+// (from about N / 2 on), and until there are enough for the partial volume,
+// whose one reduction a cell tips it back for gauss_2.  Plane over tile time,
+// d7 (14 slices a particle), slices in brackets:
+//   gauss_2    N = 384 .36 [14]  .77 [266]  .83 [518]   .82 [1792]
+//              N = 432 .33       .82        .95 (c1 .98 [512])  .88
+//              N = 480 .32       .85        1.00 (c1 1.04)      .90
+//              N = 560 .34       .92        1.07        .93
+//              N = 640 .35       .93        1.11        .93
+//   trilinear  N = 384 .42       .84        .97         .97
+//              N = 416 .39       .87        .99         1.01
+//              N = 480 .37       .90        1.05        1.04
+//              N = 640 .36       .96        1.14        1.02
 int default_tile(int mode, int N, int nsym, int np) {
-  (void)nsym; (void)np;
-  return effective_tile(kPlaneTile, mode, N);   // unless the autotuner measured otherwise
+  if (!plane_mode(mode)) return kPixelTile;
+  const long slices = (long)np * nsym;
+  if (mode == FR_MODE_GAUSS5 || N <= (mode == FR_MODE_GAUSS2 ? 432 : 400) || 2 * slices < N)
+    return kPlaneTile;
+  return mode == FR_MODE_GAUSS2 && plane_partial(N, slices) ? kPlaneTile : kPixelTile;
 }
 
 }  // namespace fr
@@ -195,11 +212,11 @@ static bool is_plane_group(int tile) { return tile >= kPlaneGroup; }
 // Each job's schedule: the caller's pin, else the autotuner's measurement for
 // its (N, mode, nsym), else the default kernel of its mode.  Jobs that share
 // a schedule share one persistent launch per round.
-static int job_tile(const fr_recon *r, int tile_pref) {
+static int job_tile(const fr_recon *r, int np, int tile_pref) {
   int t = tile_pref != -1 ? tile_pref : tuned_tile(r->N, r->mode, r->nsym);
-  if (t == -1) t = default_tile(r->mode, r->N, r->nsym, 0);
-  t = effective_tile(t, r->mode, r->N);
-  if (t == kPlaneTile || (t == kTunedScatter && plane_mode(r->mode))) return kPlaneGroup + r->mode;
+  if (t == -1) t = default_tile(r->mode, r->N, r->nsym, np);
+  t = effective_tile(t, r->mode);
+  if (t == kPlaneTile || (t == kScatterTile && plane_mode(r->mode))) return kPlaneGroup + r->mode;
   return t;
 }
 
@@ -208,8 +225,8 @@ static int job_tile(const fr_recon *r, int tile_pref) {
 static void plan_add(RoundPlan &P, fr_recon *r, int owner, int np, int tile_pref,
                      const float2 *slices, const float *t3d, const float *pw) {
   InsertJob J = make_job(r, slices, t3d, pw, np);
-  const int tile = job_tile(r, tile_pref);
-  if (tile != kTunedScatter && !is_plane_group(tile) && r->tiles_tile != tile) {
+  const int tile = job_tile(r, np, tile_pref);
+  if (tile != kScatterTile && !is_plane_group(tile) && r->tiles_tile != tile) {
     if (is_column(tile))
       column_tiles(r->N, r->mode, r->p.corners, r->tiles, r->tx, r->ty, r->tz, &r->tile_dist);
     else gather_tiles(r->N, r->mode, tile, r->p.corners, r->tiles, r->tx, r->ty, r->tz);
@@ -299,7 +316,7 @@ static void plan_groups(const std::vector<fr_recon *> &jobs, RoundPlan &P) {
       P.groups.push_back(g);
       continue;
     }
-    if (tile == kTunedScatter) {
+    if (tile == kScatterTile) {
       plan_units(P, g, false);
       P.groups.push_back(g);
       continue;
@@ -386,7 +403,7 @@ static int plan_launch_group(const RoundPlan &P, BatchScratch &bs, size_t gi, cu
   const RoundGroup &g = P.groups[gi];
   int *counter = bs.d_counter.as<int>() + gi;
   const int2 *units = (const int2 *)((const unsigned char *)bs.d_work.p + g.units_off);
-  if (g.tile == kTunedScatter) {
+  if (g.tile == kScatterTile) {
     CU(launch_scatter_multi(d_jobs, units, (int)g.nunits, g.max_px, false, st));
     return FR_OK;
   }
@@ -975,7 +992,7 @@ int fr_batch_get_accumulators(fr_batch *b, int job, float *data, float *norm) {
 }
 
 int fr_set_tile(int N, int mode, int nsym, int tile) {
-  if (tile != kTunedScatter && (tile < -1 || tile > kPixelTile))
+  if (tile != kScatterTile && (tile < -1 || tile > kPixelTile))
     return fail(FR_EINVAL_PARAM, "tile %d out of range", tile);
   std::lock_guard<std::mutex> lk(g_tune_mu);
   if (tile == -1) g_tuned.erase(std::make_tuple(N, mode, nsym));
@@ -987,8 +1004,8 @@ int fr_set_tile(int N, int mode, int nsym, int tile) {
 // schedule, on random slices of size N through random orientations; records
 // the fastest for (N, mode, nsym).  tile_out: chosen tile (-2 = scatter);
 // ms_out[kPixelTile+2]: per-candidate milliseconds (register tiles 0-3,
-// staged column 4, the mode's default kernel 5 and 6 (gauss_5: 6 is -1), then
-// scatter).
+// staged column 4, plane columns 5, pixel-major 6, then scatter; -1: not run,
+// as 6 of gauss_5 and 5 of nearest_neighbor, which have no such kernel).
 int fr_autotune(int N, int mode, int nsym, int nparticles, int *tile_out, float *ms_out) {
   if (nparticles <= 0) return fail(FR_EINVAL_PARAM, "nparticles must be positive");
   fr_params p;
@@ -1022,7 +1039,7 @@ int fr_autotune(int N, int mode, int nsym, int nparticles, int *tile_out, float 
     m[8] = (float)(e0 * e0 - e1 * e1 - e2 * e2 + e3 * e3);
   }
   float best = 1e30f;
-  int best_tile = kTunedScatter;
+  int best_tile = kScatterTile;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -1039,7 +1056,7 @@ int fr_autotune(int N, int mode, int nsym, int nparticles, int *tile_out, float 
   int measured = 0;
   for (int cand = 0; cand <= kPixelTile + 1 && rc == FR_OK; cand++) {
     const bool scatter = cand == kPixelTile + 1;
-    if (cand == kPixelTile && mode == FR_MODE_GAUSS5) {   // 5 has run it
+    if (!scatter && effective_tile(cand, mode) != cand) {   // the mode has no such kernel
       if (ms_out) ms_out[cand] = -1.0f;
       continue;
     }
@@ -1065,7 +1082,7 @@ int fr_autotune(int N, int mode, int nsym, int nparticles, int *tile_out, float 
       measured++;
     }
     if (ms_out) ms_out[cand] = ms;
-    if (ms >= 0 && ms < best) { best = ms; best_tile = scatter ? kTunedScatter : cand; }
+    if (ms >= 0 && ms < best) { best = ms; best_tile = scatter ? kScatterTile : cand; }
   }
   if (rc == FR_OK && measured == 0) rc = fail(FR_ECUDA, "autotune: no schedule ran");
   ds.release();

@@ -327,9 +327,17 @@ size_t norm_floats(int N);
 size_t slice_floats(int N);
 
 // Tile choice for the gather schedule (fr_batch.cu): measured choice when the
-// autotuner has one for (N, mode, nsym), else a size-based default.
+// autotuner has one for (N, mode, nsym), else a default by mode, size and slices.
 int tuned_tile(int N, int mode, int nsym);
 int default_tile(int mode, int N, int nsym, int np);
+// The schedule and kernel (a tile id, or kScatterTile for one thread per pixel)
+// of an insertion call (fr_api.cu).  plain: no per-pixel weights; tile: a pinned
+// id, or -1.
+struct Route {
+  bool gather;
+  int kernel;
+};
+Route insertion_route(int mode, int N, int NZ, int nsym, int np, int schedule, bool plain, int tile);
 
 }  // namespace fr
 

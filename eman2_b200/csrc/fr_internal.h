@@ -135,13 +135,13 @@ cudaError_t launch_column(const InsertJob *d_jobs, const int4 *d_work, int nwork
                           int *d_counter, int max_mode, cudaStream_t st);
 void column_tiles(int N, int mode, int corners, std::vector<int> &out, int &tx, int &ty, int &tz,
                   std::vector<float> *dist = nullptr);
-// The plane-column kernel (fr_plane.cu): gauss_5, and gauss_2 and trilinear up
-// to the size effective_tile states; of all three, every call of the scatter
-// schedule.
+// The plane-column kernel (fr_plane.cu): gauss_5, gauss_2 and trilinear; of all
+// three, every call of the scatter schedule.
 constexpr int kPlaneTile = kNumTiles + 1;
-// The pixel-major kernel: nearest_neighbor, and gauss_2 and trilinear beyond
-// that size.
+// The pixel-major kernel: nearest_neighbor, gauss_2 and trilinear (default_tile
+// says which calls).
 constexpr int kPixelTile = kNumTiles + 2;
+constexpr int kScatterTile = -2;   // the scatter, where a tile id is asked for
 inline bool plane_mode(int mode) { return mode == 2 || mode == 5 || mode == 6; }
 cudaError_t launch_plane(const InsertJob &j, cudaStream_t st);
 // The same with caller-supplied exp table and Gaussian factor.
@@ -193,17 +193,13 @@ cudaError_t launch_merge_centre(const InsertJob *d_jobs, int njobs, const Insert
 cudaError_t launch_merge(const InsertJob &j, cudaStream_t st);
 cudaError_t launch_pixel(const InsertJob *d_jobs, const int4 *d_work, int nwork, int block,
                          int *d_counter, int maxN, cudaStream_t st);
-// The kernel a job of this mode and size runs for a requested tile id.  The
-// two-tap windows' runs are short, so far beyond the L2 cache the plane-column
-// kernel waits for memory on every run, while the tile kernel adds to a tile
-// many times before it flushes it.  gauss_2, d7, plane against tile, us a
-// particle: N = 288 21.6, 26.2; N = 384 35.4, 42.8 (37 particles 43.6, 47.0);
-// N = 480 62, 68 (32 particles 81, 75); N = 640 117, 121 (32 160, 137).
-// trilinear, N = 384 42.2, 42.4.
-inline int effective_tile(int tile, int mode, int N) {
-  if (tile != kPlaneTile && tile != kPixelTile) return tile;
-  const int most = mode == 5 ? INT_MAX : (mode == 2 ? 432 : 352);
-  return plane_mode(mode) && N <= most ? kPlaneTile : kPixelTile;
+// The kernel that runs for a requested tile id: the one it names, where the
+// mode has it (gauss_5 has no pixel-major kernel, nearest_neighbor no plane
+// columns).
+inline int effective_tile(int tile, int mode) {
+  if (tile == kPlaneTile && !plane_mode(mode)) return kPixelTile;
+  if (tile == kPixelTile && mode == 5 /* gauss_5 */) return kPlaneTile;
+  return tile;
 }
 // The kernels over 16^3 tiles and slice blocks (int4 work items).
 inline bool is_column_tile(int tile) { return tile == kColumnTile || tile == kPixelTile; }

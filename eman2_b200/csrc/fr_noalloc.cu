@@ -162,7 +162,8 @@ extern "C" int fr_insert_slices_noalloc(const float *d_slices, int n, int N, int
   volatile float i2g = (float)(4.0 / (M_PI * M_PI));
   volatile float i5g = (float)(10.4 / (M_PI * M_PI));
   const float h = mode == FR_MODE_GAUSS5 ? 1.0f / i5g : 1.0f / i2g;
-  CU(plane_mode(mode) ? launch_plane_tables(j, scr + kExpOff, h, st)
-                      : launch_scatter_tables(j, scr + kExpOff, h, st));
+  const bool plane = plane_mode(mode) && !plane_small(mode, N, (long)n * nsym);
+  CU(plane ? launch_plane_tables(j, scr + kExpOff, h, st)
+           : launch_scatter_tables(j, scr + kExpOff, h, st));
   return FR_OK;
 }

@@ -856,7 +856,6 @@ static cudaError_t launch_t(const InsertJob &j, float h, const float *table, cud
 cudaError_t launch_plane_tables(const InsertJob &j, const float *table, float h, cudaStream_t st) {
   const long slices = (long)j.np * j.nsym;
   if (slices == 0) return cudaSuccess;
-  if (plane_small(j.mode, j.N, slices)) return launch_scatter_tables(j, table, h, st);
   switch (j.mode) {
     case MODE_GAUSS2: return launch_t<MODE_GAUSS2>(j, h, table, st);
     case MODE_GAUSS5: return launch_t<MODE_GAUSS5>(j, h, table, st);

@@ -344,13 +344,16 @@ FR_API int fr_batch_get_accumulators(fr_batch *b, int job, float *data, float *n
 /* Schedule selection for the insertion, measured on the device with
  * nparticles random slices and cached per (N, mode, nsym): candidates are the
  * register-tile gather shapes 0-3, the staged column kernel (4), the
- * mode's default kernel (5, and once more as 6; not for gauss_5) and the
- * scatter schedule (tile_out = -2).
+ * plane-column kernel (5; not for nearest_neighbor), the pixel-major kernel
+ * (6; not for gauss_5) and the scatter schedule (tile_out = -2).
  * ms_out, if not NULL, receives 8 timings in that order (-1: not run).  fr_set_tile pins a
- * choice (-1 clears it).  No counterpart in the reference. */
+ * choice (-1 clears it).  fr_insertion_kernel: the id of the kernel that n
+ * slices of a cubic job take now under a schedule (FR_SCHED_*; -2: one thread
+ * per pixel).  No counterpart in the reference. */
 FR_API int fr_autotune(int N, int mode, int nsym, int nparticles, int *tile_out,
                        float *ms_out);
 FR_API int fr_set_tile(int N, int mode, int nsym, int tile);
+FR_API int fr_insertion_kernel(int N, int mode, int nsym, int n, int schedule);
 
 /* Decodes n raw image values of MRC mode `mode` (0 unsigned bytes, 17 signed
  * bytes, 101 packed 4-bit, 1 int16, 6 uint16, 12 float16, 2 float32; swap:
