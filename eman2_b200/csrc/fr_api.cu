@@ -104,7 +104,7 @@ static void build_steps(float h, float K, float rmax, const float *tab, ExpSteps
   out.K = K;
   out.rout = rout;
   out.nbins = nb;
-  cudaMalloc(&out.d_bins, sizeof(float4) * nb);
+  device_malloc((void **)&out.d_bins, sizeof(float4) * nb);
   cudaMemcpy(out.d_bins, bins.data(), sizeof(float4) * nb, cudaMemcpyHostToDevice);
 }
 
@@ -118,9 +118,9 @@ Consts &consts() {
   // Util::fast_exp table (libEM/util.cpp:793): (float)exp(-i/50.0).
   float tab[1000];
   for (int i = 0; i < 1000; i++) tab[i] = (float)std::exp(-i / 50.0);
-  cudaMalloc(&c.d_exp, sizeof tab);
+  device_malloc((void **)&c.d_exp, sizeof tab);
   cudaMemcpy(c.d_exp, tab, sizeof tab, cudaMemcpyHostToDevice);
-  cudaMalloc(&c.d_err, sizeof(int));
+  device_malloc((void **)&c.d_err, sizeof(int));
   cudaMemset(c.d_err, 0, sizeof(int));
   // h = 1.0f / EMConsts::I2G and 1.0f / EMConsts::I5G (libEM/emobject.cpp:53-56,
   // libEM/reconstructor_tools.cpp:152,344).
@@ -182,12 +182,12 @@ Geom *get_geom(int N, int corners) {
   g->npix = npix;
   std::vector<float> rtab(N + 2);
   for (int i = -n2; i <= n2 + 1; i++) rtab[i + n2] = (float)i / (float)N;
-  cudaMalloc(&g->d_xmax, sizeof(int) * N);
+  device_malloc((void **)&g->d_xmax, sizeof(int) * N);
   cudaMemcpy(g->d_xmax, g->xmax.data(), sizeof(int) * N, cudaMemcpyHostToDevice);
-  cudaMalloc(&g->d_rtab, sizeof(float) * (N + 2));
+  device_malloc((void **)&g->d_rtab, sizeof(float) * (N + 2));
   cudaMemcpy(g->d_rtab, rtab.data(), sizeof(float) * (N + 2), cudaMemcpyHostToDevice);
   g->nrim = (int)rim.size();
-  cudaMalloc(&g->d_rim, sizeof(int) * std::max<size_t>(1, rim.size()));
+  device_malloc((void **)&g->d_rim, sizeof(int) * std::max<size_t>(1, rim.size()));
   if (!rim.empty())
     cudaMemcpy(g->d_rim, rim.data(), sizeof(int) * rim.size(), cudaMemcpyHostToDevice);
   m[key] = g;
@@ -461,24 +461,22 @@ int run_scatter(const InsertJob &j0, bool edge_only, cudaStream_t st) {
   return FR_OK;
 }
 
-void PlaneBufs::ensure(int N, long slices, cudaStream_t st) {
-  int half, copies;
-  centre.ensure_zero(plane_centre(N, slices, half, copies), st);
-  if (plane_partial(N, slices)) quad.ensure_zero(norm_floats(N) * sizeof(float4), st);
+size_t plane_quad_bytes(int N, long slices) {
+  return plane_partial(N, slices) ? norm_floats(N) * sizeof(float4) : 0;
 }
 
-int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st) {
+int run_plane(const InsertJob &j0, const ZeroBuf &centre, float4 *quad, cudaStream_t st) {
   const long slices = (long)j0.np * j0.nsym;
   const int N = j0.N;
   InsertJob j = j0;
   int half;
   const size_t cbytes = plane_centre(N, slices, half, j.copies);
-  if (cbytes && b.centre.cap >= cbytes) {
-    j.cdata = b.centre.as<float>();
+  if (cbytes && centre.cap >= cbytes) {
+    j.cdata = centre.as<float>();
     j.centre = half;
   }
-  const bool part = plane_partial(N, slices) && b.quad.cap >= norm_floats(N) * sizeof(float4);
-  if (part) j.quad = b.quad.as<float4>();
+  const bool part = quad && plane_partial(N, slices);
+  if (part) j.quad = quad;
   const long turns = part || j.cdata ? (slices + kPlaneTurn - 1) / kPlaneTurn : 1;
   const int per = (int)((j0.np + turns - 1) / turns);
   for (int p0 = 0; p0 < j0.np; p0 += per) {
@@ -547,8 +545,12 @@ int insert_device(fr_recon *r, const float2 *d_slices, const float *d_t3d, const
   if (plane || tile == kScatterTile) {
     if (prof) CU(cudaEventRecord(ev[0], st));
     if (plane) {
-      r->plane.ensure(r->N, (long)np * r->nsym, st);
-      TRY(run_plane(j, r->plane, st));
+      const long slices = (long)np * r->nsym;
+      int half, copies;
+      r->centre.ensure_zero(plane_centre(r->N, slices, half, copies), st);
+      PlaneLease lease(plane_quad_bytes(r->N, slices), st);
+      TRY(run_plane(j, r->centre, lease.quad(), st));
+      TRY(lease.done());
     } else {
       TRY(run_scatter(j, false, st));
     }
@@ -915,9 +917,8 @@ int fr_destroy(fr_recon *r) {
                       &r->s_meta, &r->ref,
                       &r->s_w, &r->s_t3d, &r->s_img, &r->s_img2, &r->s_spec, &r->s_ctf,
                       &r->s_txy, &r->s_out, &r->s_ssnr, &r->s_jobs, &r->s_work,
-                      &r->s_counter};
+                      &r->s_counter, &r->centre};
     for (DevBuf *b : bufs) b->release();
-    r->plane.release();
     for (int k = 0; k < 2; k++) {
       r->s_stage[k].release();
       if (r->staged[k]) cudaEventDestroy(r->staged[k]);

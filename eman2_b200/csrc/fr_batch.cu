@@ -81,12 +81,23 @@ struct ProBufs {
   }
 };
 
+// A schedule group's plane workspaces: the centre copies, and for a captured
+// graph, whose branches run side by side on addresses of their own, a partial
+// volume (a call borrows the device's, PlaneLease).
+struct PlaneBufs {
+  ZeroBuf centre, quad;
+  void release() {
+    centre.release();
+    quad.release();
+  }
+};
+
 // Device copies of a batched launch's job table and work list, the round's
 // metadata block and the prologue groups' scratch.
 struct BatchScratch {
   DevBuf d_jobs, d_work, d_counter, d_meta;
   std::vector<ProBufs> gbufs;
-  std::vector<PlaneBufs> plane;   // per schedule group (groups may run concurrently)
+  std::vector<PlaneBufs> plane;   // per schedule group
   PinnedRing ring;
   cudaEvent_t done = nullptr;     // after the last launch that read this scratch
   cudaStream_t last = nullptr;
@@ -372,8 +383,9 @@ static void plan_groups(const std::vector<fr_recon *> &jobs, RoundPlan &P) {
 // vectors: the copies have taken them when cudaMemcpyAsync returns), and the
 // plane groups' workspaces.  The centre copies of a group's shared launch sit
 // one after another; a job that takes turns by itself has all of its own
-// before or after, so it reuses them from the start.
-static int plan_upload(RoundPlan &P, BatchScratch &bs, cudaStream_t st) {
+// before or after, so it reuses them from the start.  captured: the groups get
+// partial volumes of their own.
+static int plan_upload(RoundPlan &P, BatchScratch &bs, cudaStream_t st, bool captured) {
   TRY(bs.d_jobs.ensure(sizeof(InsertJob) * std::max<size_t>(1, P.hj.size())));
   TRY(bs.d_counter.ensure(sizeof(int) * std::max<size_t>(1, P.groups.size())));
   TRY(bs.d_work.ensure(std::max<size_t>(16, P.work.size())));
@@ -381,7 +393,13 @@ static int plan_upload(RoundPlan &P, BatchScratch &bs, cudaStream_t st) {
   for (size_t gi = 0; gi < P.groups.size(); gi++) {
     RoundGroup &g = P.groups[gi];
     PlaneBufs &b = bs.plane[gi];
-    for (int k : g.turns) b.ensure(P.hj[k].N, (long)P.hj[k].np * P.hj[k].nsym, st);
+    for (int k : g.turns) {
+      const InsertJob &J = P.hj[k];
+      const long slices = (long)J.np * J.nsym;
+      int half, copies;
+      b.centre.ensure_zero(plane_centre(J.N, slices, half, copies), st);
+      if (captured) b.quad.ensure_zero(plane_quad_bytes(J.N, slices), st);
+    }
     if (!b.centre.ensure_zero(g.centre_bytes, st)) g.centres.clear();
     for (const auto &c : g.centres) {
       InsertJob &J = P.hj[c.first];
@@ -397,8 +415,9 @@ static int plan_upload(RoundPlan &P, BatchScratch &bs, cudaStream_t st) {
 // Device work of schedule group gi: one persistent launch (or the scatter
 // over all its jobs), then the face taps.  Kernels only; each group has its
 // own work counter, so groups (which insert into different jobs) may run
-// concurrently.
-static int plan_launch_group(const RoundPlan &P, BatchScratch &bs, size_t gi, cudaStream_t st) {
+// concurrently, unless they share a partial volume (lent; null: their own).
+static int plan_launch_group(const RoundPlan &P, BatchScratch &bs, size_t gi, cudaStream_t st,
+                             float4 *lent) {
   const InsertJob *d_jobs = bs.d_jobs.as<InsertJob>();
   const RoundGroup &g = P.groups[gi];
   int *counter = bs.d_counter.as<int>() + gi;
@@ -408,7 +427,12 @@ static int plan_launch_group(const RoundPlan &P, BatchScratch &bs, size_t gi, cu
     return FR_OK;
   }
   if (is_plane_group(g.tile)) {
-    for (int k : g.turns) TRY(run_plane(P.hj[k], bs.plane[gi], st));
+    const PlaneBufs &b = bs.plane[gi];
+    for (int k : g.turns) {
+      const InsertJob &J = P.hj[k];
+      const bool own = b.quad.cap >= plane_quad_bytes(J.N, (long)J.np * J.nsym);
+      TRY(run_plane(J, b.centre, lent ? lent : own ? b.quad.as<float4>() : nullptr, st));
+    }
     CU(launch_plane_multi(d_jobs, (const PlaneSeg *)units, (int)g.nunits, g.units, g.max_mode,
                           g.maxN, g.patches, st));
     if (!g.centres.empty())
@@ -428,9 +452,18 @@ static int plan_launch_group(const RoundPlan &P, BatchScratch &bs, size_t gi, cu
 }
 
 // The round's schedule groups one after another on st.
-static int plan_launch(const RoundPlan &P, BatchScratch &bs, cudaStream_t st) {
-  for (size_t gi = 0; gi < P.groups.size(); gi++) TRY(plan_launch_group(P, bs, gi, st));
+static int plan_launch(const RoundPlan &P, BatchScratch &bs, cudaStream_t st, float4 *lent) {
+  for (size_t gi = 0; gi < P.groups.size(); gi++) TRY(plan_launch_group(P, bs, gi, st, lent));
   return FR_OK;
+}
+
+// Bytes of the partial volume that the round's jobs take turns at.
+static size_t plan_quad_bytes(const RoundPlan &P) {
+  size_t most = 0;
+  for (const RoundGroup &g : P.groups)
+    for (int k : g.turns)
+      most = std::max(most, plane_quad_bytes(P.hj[k].N, (long)P.hj[k].np * P.hj[k].nsym));
+  return most;
 }
 
 // ------------------------------------------------------------ prologue groups
@@ -609,8 +642,10 @@ static int batch_insert(std::vector<fr_recon *> &jobs, BatchScratch &bs, int til
       TRY(group_run(jobs, G[gi], bs.gbufs[gi], bs.d_meta.as<unsigned char>() + G[gi].meta_off, &P,
                     tile_pref, st));
     plan_groups(jobs, P);
-    TRY(plan_upload(P, bs, st));
-    TRY(plan_launch(P, bs, st));
+    TRY(plan_upload(P, bs, st, false));
+    PlaneLease lease(plan_quad_bytes(P), st);
+    TRY(plan_launch(P, bs, st, lease.quad()));
+    TRY(lease.done());
   }
   CU(cudaEventRecord(bs.done, st));
   bs.last = st;
@@ -733,12 +768,12 @@ static int graph_device_work(fr_graph *g, cudaStream_t st) {
     }
   // the schedule groups (disjoint jobs) as parallel branches too
   const int nsched = (int)g->plan.groups.size();
-  if (nsched <= 1) return plan_launch(g->plan, g->bs, st);
+  if (nsched <= 1) return plan_launch(g->plan, g->bs, st, nullptr);
   const int nside2 = std::min(nsched, (int)fr_graph::kSide);
   CU(cudaEventRecord(g->fork, st));
   for (int k = 0; k < nside2; k++) CU(cudaStreamWaitEvent(g->side[k], g->fork, 0));
   for (int gi = 0; gi < nsched; gi++)
-    TRY(plan_launch_group(g->plan, g->bs, gi, g->side[gi % fr_graph::kSide]));
+    TRY(plan_launch_group(g->plan, g->bs, gi, g->side[gi % fr_graph::kSide], nullptr));
   for (int k = 0; k < nside2; k++) {
     CU(cudaEventRecord(g->join[k], g->side[k]));
     CU(cudaStreamWaitEvent(st, g->join[k], 0));
@@ -855,7 +890,7 @@ static int graph_create(const std::vector<fr_recon *> &jobs, cudaStream_t st, in
                    true);
   if (rc == FR_OK) {
     plan_groups(jobs, g->plan);
-    rc = plan_upload(g->plan, g->bs, st);
+    rc = plan_upload(g->plan, g->bs, st, true);
   }
   if (rc == FR_OK && cudaStreamSynchronize(st) != cudaSuccess)
     rc = fail(FR_ECUDA, "sizing pass failed: %s", cudaGetErrorString(cudaGetLastError()));

@@ -44,6 +44,13 @@ inline bool same_stream(cudaStream_t before, cudaStream_t now) {
   return before == now && now != cudaStreamPerThread;
 }
 
+// cudaMalloc that, finding no room, takes back what the library can spare
+// (fr_workspace.cu) and tries again.
+cudaError_t device_malloc(void **p, size_t bytes);
+// Gives the device's idle shared workspace back; whether there was one.
+bool reclaim_device_memory();
+void workspace_leave();   // no handle is left
+
 struct DevBuf {
   void *p = nullptr;
   size_t cap = 0;
@@ -52,7 +59,7 @@ struct DevBuf {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    if (device_malloc(&p, bytes) != cudaSuccess) {
       cudaGetLastError();
       return fail(FR_ENOMEM, "device allocation of %zu bytes failed", bytes);
     }
@@ -67,10 +74,10 @@ struct DevBuf {
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
-// Workspaces the plane kernel inserts into and its merges clear again (a
-// partial volume; copies of the cells near the origin): zero between launches,
-// whatever sizes shared them.  Without memory for them the insertion goes
-// straight to the accumulators.
+// Workspaces the plane kernel inserts into and its merges clear again (copies
+// of the cells near the origin, at most 6 MB a job; a captured graph's partial
+// volume): zero between launches, whatever sizes shared them.  Without memory
+// for them the insertion goes straight to the accumulators.
 struct ZeroBuf : DevBuf {
   // Whether the buffer holds at least `bytes`, zeroed on st when it grew.
   bool ensure_zero(size_t bytes, cudaStream_t st) {
@@ -81,13 +88,24 @@ struct ZeroBuf : DevBuf {
     return false;
   }
 };
-struct PlaneBufs {
-  ZeroBuf quad, centre;
-  // Makes room for a call (plane_partial, plane_centre decide what it uses).
-  void ensure(int N, long slices, cudaStream_t st);
-  void release() {
-    for (DevBuf *b : {(DevBuf *)&quad, (DevBuf *)&centre}) b->release();
-  }
+
+// A call's turn at the device's shared partial volume (fr_workspace.cu), from
+// its construction to done(), which says that the work queued on st since
+// leaves it zero.  Without done() the volume is given up.
+class PlaneLease {
+ public:
+  PlaneLease(size_t bytes, cudaStream_t st);
+  ~PlaneLease();
+  PlaneLease(const PlaneLease &) = delete;
+  PlaneLease &operator=(const PlaneLease &) = delete;
+  float4 *quad() const { return quad_; }   // null: no room (or 0 bytes asked for)
+  int done();
+
+ private:
+  void give_back(bool clean);
+  void *shared_ = nullptr;
+  float4 *quad_ = nullptr;
+  cudaStream_t st_;
 };
 
 // Pinned host staging for per-call uploads (metadata blocks, job tables,
@@ -235,7 +253,13 @@ struct PlanCache {
   int make3d(cufftHandle *h, int nz, int ny, int nx, cufftType type) {
     TRY(fresh(h));
     size_t ws = 0;
-    const cufftResult r = cufftMakePlan3d(*h, nz, ny, nx, type, &ws);
+    cufftResult r = cufftMakePlan3d(*h, nz, ny, nx, type, &ws);
+    if (r == CUFFT_ALLOC_FAILED && reclaim_device_memory()) {
+      cudaGetLastError();
+      cufftDestroy(*h);
+      TRY(fresh(h));
+      r = cufftMakePlan3d(*h, nz, ny, nx, type, &ws);
+    }
     if (r != CUFFT_SUCCESS) {
       cufftDestroy(*h);
       *h = 0;
@@ -277,11 +301,19 @@ struct PlanCache {
       int n[2] = {N, N};
       const int dist_r = N * N, dist_c = N * (N / 2 + 1);
       size_t ws = 0;
-      const cufftResult r =
-          forward ? cufftMakePlanMany(h, 2, n, nullptr, 1, dist_r, nullptr, 1, dist_c, CUFFT_R2C,
-                                      batch, &ws)
-                  : cufftMakePlanMany(h, 2, n, nullptr, 1, dist_c, nullptr, 1, dist_r, CUFFT_C2R,
-                                      batch, &ws);
+      auto make = [&] {
+        return forward ? cufftMakePlanMany(h, 2, n, nullptr, 1, dist_r, nullptr, 1, dist_c,
+                                           CUFFT_R2C, batch, &ws)
+                       : cufftMakePlanMany(h, 2, n, nullptr, 1, dist_c, nullptr, 1, dist_r,
+                                           CUFFT_C2R, batch, &ws);
+      };
+      cufftResult r = make();
+      if (r == CUFFT_ALLOC_FAILED && reclaim_device_memory()) {
+        cudaGetLastError();
+        cufftDestroy(h);
+        TRY(fresh(&h));
+        r = make();
+      }
       if (r != CUFFT_SUCCESS) {
         cufftDestroy(h);
         return fail(r == CUFFT_ALLOC_FAILED ? FR_ENOMEM : FR_ECUDA,
@@ -360,7 +392,7 @@ struct fr_recon {
   // scratch
   fr::DevBuf s_in, s_slices, s_rot, s_w, s_t3d, s_img, s_img2, s_spec, s_ctf, s_txy, s_out,
       s_ssnr, s_jobs, s_work, s_counter;
-  fr::PlaneBufs plane;
+  fr::ZeroBuf centre;         // the plane kernel's centre copies
   fr::PlanCache plans;
   int tile = -1;              // gather tile shape (-1: tuned default)
   std::vector<int> tiles;
@@ -412,10 +444,12 @@ int stream_leave_all(const std::vector<fr_recon *> &rs, cudaStream_t st,
                      std::shared_ptr<SharedEvent> *reuse = nullptr);
 InsertJob make_job(fr_recon *r, const float2 *slices, const float *t3d, const float *pw, int np);
 int run_scatter(const InsertJob &j0, bool edge_only, cudaStream_t st);
-// The plane-column insertion of one job: through the partial volume in turns
-// of kPlaneTurn slices when the call is large enough (plane_partial), with
-// centre copies from 16 slices on, as far as `b` has room for them.
-int run_plane(const InsertJob &j0, const PlaneBufs &b, cudaStream_t st);
+// Bytes of the partial volume of a call of so many slices (0: it takes none).
+size_t plane_quad_bytes(int N, long slices);
+// The plane-column insertion of one job: through the partial volume `quad`
+// (plane_quad_bytes; null: none) in turns of kPlaneTurn slices, with centre
+// copies from 16 slices on if `centre` has room for them.
+int run_plane(const InsertJob &j0, const ZeroBuf &centre, float4 *quad, cudaStream_t st);
 int insert_device(fr_recon *r, const float2 *d_slices, const float *d_t3d, const float *d_pw, int np,
                   int schedule, const float *d_ssnr, int nssnr);
 int check_device_error(fr_recon *r);

@@ -95,6 +95,7 @@ bool one_thread(unsigned char *pinned, unsigned char *dst, const unsigned char *
 void host_pool_enter() { g_handles++; }
 void host_pool_leave() {
   if (--g_handles > 0) return;
+  workspace_leave();
   std::lock_guard<std::mutex> lk(g_pool.use);
   if (g_handles > 0 || !g_pool.p) return;
   cudaFreeHost(g_pool.p);

@@ -549,7 +549,7 @@ static int get_plan(int N, Plan &out) {
   }
   unsigned char *d = nullptr;
   const size_t tb = sizeof(float2) * N;
-  if (cudaMalloc(&d, tb + sizeof(short) * N) != cudaSuccess) {
+  if (device_malloc((void **)&d, tb + sizeof(short) * N) != cudaSuccess) {
     cudaGetLastError();
     return fail(FR_ENOMEM, "device allocation of %zu bytes failed", tb + sizeof(short) * N);
   }

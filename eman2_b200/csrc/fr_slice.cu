@@ -590,7 +590,7 @@ static int slice_twiddles(int N, const float2 **out) {
       h[i] = make_float2((float)std::cos(w), (float)std::sin(w));
     }
     float2 *d = nullptr;
-    if (cudaMalloc(&d, sizeof(float2) * N) != cudaSuccess) {
+    if (device_malloc((void **)&d, sizeof(float2) * N) != cudaSuccess) {
       cudaGetLastError();
       return fail(FR_ENOMEM, "device allocation of %zu bytes failed", sizeof(float2) * N);
     }

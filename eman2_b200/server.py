@@ -57,7 +57,9 @@ def footprint_bytes(params: dict, box: int, chunk: int) -> int:
     """Device bytes a job holds: the (complex, weight) accumulators
     (12*(N/2+1)*N^2 bytes, as libEM/reconstructor.cpp:782,800 allocate) plus
     the per-chunk prologue and slice scratch (~5 N^2 floats per particle and
-    the raw images)."""
+    the raw images).  The partial volume of large insertions is no job's: the
+    device's jobs share one, and the library gives it back when an allocation
+    finds no room."""
     N = int(params["size"][0]) if not np.isscalar(params["size"]) else int(params["size"])
     vol = 4 * (N * N * (N + 2) + N * N * (N // 2 + 1))
     return vol + chunk * (20 * N * N + 4 * box * box)

@@ -206,6 +206,11 @@ FR_API int fr_get_accumulators(fr_recon *r, float *data, float *norm);
 
 /* Sizes and state. */
 FR_API int fr_get_size(const fr_recon *r, int *N);
+/* Device bytes of a job's accumulators.  Beside them large insertions of all
+ * of a device's handles take turns at one workspace of 16 bytes per cell of the
+ * largest volume (4/3 of its accumulators): no job holds it, it is taken only
+ * where it leaves a quarter of the free memory, and the library gives it back
+ * when one of its allocations finds no room and with the last handle. */
 FR_API size_t fr_footprint_bytes(int N);
 
 /* Symmetry operators of a symmetry name (Symmetry3D::get_symmetries,
