@@ -137,6 +137,31 @@ def load_peaks():
         return 6650.0, "fallback"
 
 
+# The insertion kernels by the library's ids, and the measured update roof that
+# describes a kernel's additions: one shared read-modify-write a tap (the staged
+# column kernel, the plane columns of the two-tap windows), three shared FP32
+# atomics (the pixel-major kernel), three L2 reductions (one thread per pixel).
+# gauss_5's plane columns sum in registers and the register tiles own their
+# voxels: no measured roof is theirs.
+KERNELS = {-2: "k_scatter", 4: "k_column", 5: "k_plane", 6: "k_pixel"}
+UPDATE_ROOFS = {"smem_rmw": "shared-memory float4 read-modify-write",
+                "smem_atom": "shared-memory FP32 atomics (3 per tap)",
+                "l2_red": "L2 red.global.add.f32 (3 per tap)"}
+
+
+def insertion_kernel_name(wl, n: int, schedule: str = "auto") -> str:
+    """The kernel that n particles a call of this workload are inserted by."""
+    from eman2_b200.batch import insertion_kernel
+    return KERNELS.get(insertion_kernel(wl["N"], wl["mode"], nsym_of(wl["sym"]), n, schedule),
+                       "k_gather")
+
+
+def update_roof_of(kernel: str, mode: str):
+    if kernel == "k_plane":
+        return None if mode == "gauss_5" else "smem_rmw"
+    return {"k_column": "smem_rmw", "k_pixel": "smem_atom", "k_scatter": "l2_red"}.get(kernel)
+
+
 def load_traffic(workload: str, batch: int):
     """DRAM bytes (read + write) of one insertion call of this workload and
     batch (all of its launches), from the committed ncu capture of the same bench command; None
@@ -798,15 +823,16 @@ def run_target(dev, steps: int = 3, plain_n: int = 64):
     taps = nsym_of(wl["sym"]) * pixels_per_slice(N) * 8 * 2048 / (gms / 1e3)
     upd = update_peaks()
     out = {"workload": wl["desc"], "batched": {"value": batched, "unit": "particle-slices/s",
-                                               "particles_per_call": 2048, "kernel": "k_plane",
+                                               "particles_per_call": 2048,
+                                               "kernel": insertion_kernel_name(wl, 2048),
                                                "avg_launch_ms": gms},
            "plain": {"value": plain, "unit": "particle-slices/s", "sample": plain_n,
-                     "kernel": "k_scatter"},
+                     "kernel": insertion_kernel_name(wl, 1, "scatter")},
            "batched_vs_plain": batched / plain}
-    if upd is not None:
-        out["update_roofline"] = {"bound": "shared-memory float4 read-modify-write",
-                                  "achieved": taps, "peak": upd["smem_rmw"], "unit": "taps/s",
-                                  "frac": taps / upd["smem_rmw"]}
+    roof = update_roof_of(out["batched"]["kernel"], wl["mode"])
+    if upd is not None and roof:
+        out["update_roofline"] = {"bound": UPDATE_ROOFS[roof], "achieved": taps,
+                                  "peak": upd[roof], "unit": "taps/s", "frac": taps / upd[roof]}
     # the HBM roofline of the same launch, as the main line's (algorithmic
     # bytes over the launch time) with its committed DRAM traffic
     peak, peak_kind = load_peaks()
@@ -938,8 +964,8 @@ def main():
     ap.add_argument("--no-accuracy", action="store_true",
                     help="skip the accuracy leg (GPU forms against the oracles)")
     ap.add_argument("--tile", type=int, default=-1,
-                    help="pin the insertion kernel (0-3 register tiles, 4 staged column, 5 or 6 the "
-                         "mode's default kernel, -2 scatter); default: library choice")
+                    help="pin the insertion kernel (0-3 register tiles, 4 staged column, 5 plane "
+                         "columns, 6 pixel-major, -2 scatter); default: library choice")
     args = ap.parse_args()
     wl = WORKLOADS[args.workload]
     ws, rank, local = dist_setup()
@@ -983,16 +1009,13 @@ def main():
     e2e = ws * args.steps * args.batch / (e2e_ms / 1e3)
     V = (N // 2 + 1) * N * N
     alg_bytes = args.batch * (8 * (N // 2 + 1) * N + 64) + 24 * V
+    kname = insertion_kernel_name(wl, args.batch)
+    roof = update_roof_of(kname, wl["mode"])
     if st["gather_launches"] > 0:
-        # the library's default: k_plane, and k_pixel for the narrow windows of large volumes
-        most = {"gauss_5": N, "gauss_2": 432, "trilinear": 352}.get(wl["mode"], 0)
-        plane = N <= most
-        tile = args.tile if args.tile not in (-1, 5, 6) else (5 if plane else 6)
-        kname = {6: "k_pixel", 5: "k_plane", 4: "k_column"}.get(tile, "k_gather") + \
-            " (gather schedule)"
+        kname += " (gather schedule)"
         gms = st["gather_ms"] / st["gather_launches"]
     else:
-        kname, gms = "k_scatter", st["insert_ms"] / max(1, st["insert_launches"])
+        gms = st["insert_ms"] / max(1, st["insert_launches"])
     achieved = alg_bytes / (gms / 1e3) / 1e9
     peak, peak_kind = load_peaks()
     traffic = load_traffic(args.workload, args.batch)
@@ -1017,20 +1040,11 @@ def main():
         "taps": {"per_particle_upper": taps_per, "per_s_upper": taps_s},
         "clocks": clk,
     }
-    if upd is not None:
-        # the binding roof: the rate of the accumulator update the kernel
-        # uses (the column kernels: one shared read-modify-write per tap,
-        # which gauss_5's plane columns mostly save by summing in registers;
-        # the pixel kernel: three shared FP32 atomics; the scatter:
-        # three L2 reductions)
-        key = ("l2_red" if st["gather_launches"] == 0 else
-               "smem_atom" if kname.startswith("k_pixel") else "smem_rmw")
+    if upd is not None and roof:
         line["update_roofline"] = {
-            "bound": {"smem_rmw": "shared-memory float4 read-modify-write",
-                      "smem_atom": "shared-memory FP32 atomics (3 per tap)",
-                      "l2_red": "L2 red.global.add.f32 (3 per tap)"}[key],
-            "achieved": taps_s, "peak": upd[key], "unit": "taps/s", "frac": taps_s / upd[key],
-            "peaks_measured": upd, "taps": "upper bound S*p(N)*window"}
+            "bound": UPDATE_ROOFS[roof], "achieved": taps_s, "peak": upd[roof], "unit": "taps/s",
+            "frac": taps_s / upd[roof], "peaks_measured": upd,
+            "taps": "upper bound S*p(N)*window"}
     if agree is not None:
         line["agreement"] = agree
     if plain is not None:

@@ -122,3 +122,14 @@ def test_default_kernels_at_large_sizes(gpu, mode, N, sym, n, kernel):
     o.insert(sl, rots, w, mode, sym)
     assert np.array_equal(nm != 0, o.norm != 0)
     assert oracle.rel_l2(nm, o.norm) < RTOL and oracle.rel_l2(d, o.data) < RTOL
+
+
+def test_bench_names_the_kernel_that_runs():
+    import bench
+    c4, g2 = bench.WORKLOADS["c4"], bench.WORKLOADS["c4g2"]
+    assert bench.insertion_kernel_name(c4, 2048) == "k_plane"
+    assert bench.insertion_kernel_name(g2, 2048) == "k_plane"
+    assert bench.insertion_kernel_name(g2, 1, "scatter") == "k_plane"    # 14 slices of 384^2
+    assert bench.insertion_kernel_name(dict(g2, N=96, sym="c1"), 1, "scatter") == "k_scatter"
+    assert bench.update_roof_of("k_plane", "gauss_5") is None
+    assert bench.update_roof_of("k_plane", "gauss_2") == "smem_rmw"
