@@ -399,9 +399,11 @@ constexpr int kRexpCopies = 8;
 
 // Util::fast_exp(-y) for y in [0, 7.5) read from the interleaved copies.  The
 // reference's index (int)(y*50.0+0.5) is floor(50y + 1/2): one multiply-add
-// rounded down onto a spacing of 1/4 leaves it in mantissa bits 2 and up.
+// rounded down onto a spacing of 1/4 leaves it in mantissa bits 2 and up.  The
+// lookup comes before the test for taps in the tile, so a coordinate that is no
+// number, or far outside, has to end in the table too.
 __device__ __forceinline__ float rexp_lookup(float y, const float *rexp) {
-  const int t = __float_as_int(__fmaf_rd(y, 50.0f, 2097152.5f)) & 0x1FFC;
+  const int t = min(__float_as_int(__fmaf_rd(y, 50.0f, 2097152.5f)) & 0x1FFC, 4 * (kRexpEntries - 1));
   return rexp[t * (kRexpCopies / 4) + (threadIdx.x & (kRexpCopies - 1))];
 }
 

@@ -15,10 +15,11 @@ enum { MODE_NEAREST = 1, MODE_GAUSS2 = 2, MODE_GAUSS5 = 5, MODE_TRILINEAR = 6, M
 // The index is formed exactly in single precision: 50*y = p + e exactly
 // (p rounded product, e its FMA residual), so floor(50*y + 0.5) is
 // floor(p) + [frac(p) + e >= 0.5], with frac(p) exact by Sterbenz.
-// The comparison f < -19.98f selects the same floats as the double
-// comparison f < -19.98 (the float nearest 19.98 lies below it).
+// The comparison f >= -19.98f selects the same floats as the double
+// comparison f >= -19.98 (the float nearest 19.98 lies below it).  A NaN (a
+// matrix with one) is not in the table's range either.
 __device__ __forceinline__ float fast_exp(float f, const float *__restrict__ table) {
-  if (f > 0.0f || f < -19.98f) return expf(f);
+  if (!(f <= 0.0f && f >= -19.98f)) return expf(f);
   const float y = -f;
   const float p = __fmul_rn(y, 50.0f);
   const float e = __fmaf_rn(y, 50.0f, -p);
@@ -109,8 +110,10 @@ __device__ __forceinline__ void tap_value(int i, int j, int k, float xx, float y
 __device__ __forceinline__ void add_tap_atomic(float *__restrict__ data, float *__restrict__ norm,
                                                int N, int NZ, int x, int y, int z, float re,
                                                float im, float wt) {
-  const int h = N >> 1;
-  if (abs(x) > h || abs(y) > h || abs(z) > (NZ >> 1)) return;
+  const int h = N >> 1, hz = NZ >> 1;
+  // |x|, |y| <= N/2, |z| <= NZ/2 (unsigned: INT_MIN, from a coordinate beyond
+  // the integers, has no absolute value)
+  if ((unsigned)x + h > 2u * h || (unsigned)y + h > 2u * h || (unsigned)z + hz > 2u * hz) return;
   const size_t nxf = (size_t)N + 2;
   const size_t nxy = nxf * (size_t)N;
   const size_t rc = (size_t)(y <= 0 ? -y : N - y) * nxf + (size_t)(z <= 0 ? -z : NZ - z) * nxy;

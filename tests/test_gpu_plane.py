@@ -112,3 +112,42 @@ def test_small_volumes_in_one_launch(gpu, mode):
         assert np.array_equal(nm != 0, o.norm != 0)
         assert oracle.rel_l2(nm, o.norm) < RTOL and oracle.rel_l2(d, o.data) < 2e-5
     b.close()
+
+
+@pytest.mark.parametrize("tile", [5, 6, -2])
+@pytest.mark.parametrize("mode", ["gauss_2", "trilinear"])
+def test_matrices_of_no_numbers(gpu, mode, tile):
+    """Slices whose first rows hold a NaN or are scaled beyond the integers end
+    inside the kernels' tables and volumes: the call returns, and away from the
+    origin, where the NaN coordinates' taps go, the sums are the others'."""
+    from eman2_b200 import Reconstructors, _lib
+    from eman2_b200.batch import set_tile
+    N, n = 40, 60
+    rng = np.random.default_rng(8)
+    sl = rng.normal(size=(n, N, N + 2)).astype(np.float32)
+    w = np.ones(n, np.float32)
+    rots = _rotations(n, 9)
+    bad = rots.copy()
+    bad[20, 0, 1] = np.nan
+    bad[30, 1, 0] = np.nan
+    bad[40, :2] *= 1e9
+    bad[50, :2] *= 1e12
+    bad[55, 0] = np.inf
+    o = oracle.OracleVolume(N, "fp32acc64")
+    keep = np.setdiff1d(np.arange(n), [20, 30, 40, 50, 55])
+    o.insert(sl[keep], rots[keep], w[keep], mode, "c1")
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": mode})
+    r.setup()
+    set_tile(N, mode, 1, tile)
+    try:
+        r.insert_slices(sl, bad, w, schedule="scatter" if tile == -2 else "gather")
+        d, nm = r.get_accumulators()
+    finally:
+        set_tile(N, mode, 1, -1)
+    far = np.ones(nm.shape, bool)
+    near = np.r_[0:3, N - 2:N]
+    far[np.ix_(near, near, [0, 1, 2])] = False
+    assert np.isfinite(nm[far]).all()
+    assert oracle.rel_l2(nm[far], o.norm[far]) < RTOL
+    cells = nm.shape + (2,)
+    assert oracle.rel_l2(d.reshape(cells)[far], o.data.reshape(cells)[far]) < RTOL
