@@ -679,7 +679,7 @@ __device__ void tile_item4(const InsertJob &J, int tile, int s0, int s1, const S
     pixel_pass<MODE>(J, S, M, (u & 1) ? -1 : 1, base, ext, sl, w, h);
   }
   __syncthreads();
-  // ---- flush (as tile_item3)
+  // ---- flush the tile's sums into the volume; a touched origin keeps no imaginary part
   const size_t nxf = (size_t)N + 2;
   for (int i = threadIdx.x; i < NV; i += NT) {
     const int lz = i >> 8, ly = (i >> 4) & 15, lx = i & 15;
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(col::NT, 3)
       case MODE_NEAREST: col::tile_item4<MODE_NEAREST>(J, wk.y, s0, s1, S, h2, exp_g); break;
       case MODE_TRILINEAR: col::tile_item4<MODE_TRILINEAR>(J, wk.y, s0, s1, S, h2, exp_g); break;
       default:
-        if (threadIdx.x == 0) atomicOr(err, 4);   // gauss_5 takes the column kernel
+        if (threadIdx.x == 0) atomicOr(err, 4);   // gauss_5 has no pixel-major kernel
     }
   }
 }

@@ -159,8 +159,8 @@ cudaError_t launch_plane_multi(const InsertJob *d_jobs, const PlaneSeg *d_segs, 
                                int units, int mode, int maxN, long patches, cudaStream_t st);
 // Patches of columns of so many slices (about three quarters of a bounding box's).
 long plane_patches(int N, long slices);
-// A few small slices of the two-tap windows: one thread per pixel ends sooner
-// than one lane per column, which walks 5 to 6 pixels and their rows (gauss_2,
+// A few small slices of the two-tap windows, unless id 5 is pinned: one thread
+// per pixel ends sooner than one lane per column, which walks 5 to 6 pixels and their rows (gauss_2,
 // c1: N = 192 6.7 against 10.6 us, N = 384 10.8 against 13.6; with c4 24.7
 // against 29.3; with d7 68 against 58).  gauss_5 has none (N = 48, c1: 72
 // against 44 us).

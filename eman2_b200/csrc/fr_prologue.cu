@@ -8,9 +8,9 @@
 //   recon.preprocess_slice(img, ts)         (libEM/reconstructor.cpp:1022-1061):
 //     bilinear xform (libEM/processor.cpp:11025-11080), phase origin to corner,
 //     r2c FFT, x sqrt((N+2)/N)
-// Here, for sizes fr_slice.cu does not take, the FFTs are batched cuFFT plans
-// and everything between them is one kernel per stage over all particles of a
-// chunk.
+// Here, for the calls that neither fr_slice.cu nor fr_lines.cu takes, the FFTs
+// are batched cuFFT plans and everything between them is one kernel per stage
+// over all particles of a chunk.
 #include <algorithm>
 #include <cmath>
 
