@@ -110,10 +110,8 @@ __device__ __forceinline__ void tap_value(int i, int j, int k, float xx, float y
 __device__ __forceinline__ void add_tap_atomic(float *__restrict__ data, float *__restrict__ norm,
                                                int N, int NZ, int x, int y, int z, float re,
                                                float im, float wt) {
-  const int h = N >> 1, hz = NZ >> 1;
-  // |x|, |y| <= N/2, |z| <= NZ/2 (unsigned: INT_MIN, from a coordinate beyond
-  // the integers, has no absolute value)
-  if ((unsigned)x + h > 2u * h || (unsigned)y + h > 2u * h || (unsigned)z + hz > 2u * hz) return;
+  const int h = N >> 1;
+  if (abs(x) > h || abs(y) > h || abs(z) > (NZ >> 1)) return;
   const size_t nxf = (size_t)N + 2;
   const size_t nxy = nxf * (size_t)N;
   const size_t rc = (size_t)(y <= 0 ? -y : N - y) * nxf + (size_t)(z <= 0 ? -z : NZ - z) * nxy;
@@ -184,6 +182,8 @@ __device__ __forceinline__ void insert_pixel_atomic(float *__restrict__ data, fl
     const int x0 = (int)floorf(__fadd_rn(xx, 0.5f));
     const int y0 = (int)floorf(__fadd_rn(yy, 0.5f));
     const int z0 = (int)floorf(__fadd_rn(zz, 0.5f));
+    // (the least integer, from a coordinate beyond them, has no absolute value)
+    if (x0 < -n2 || y0 < -n2 || z0 < -nz2) return;
     if (face_only && abs(x0) != n2 && abs(y0) != n2 && abs(z0) != nz2) return;
     add_tap_atomic(data, norm, N, NZ, x0, y0, z0, __fmul_rn(re, w), __fmul_rn(im, w), w);
   } else if (MODE == MODE_GAUSS2 || MODE == MODE_TRILINEAR) {

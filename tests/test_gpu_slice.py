@@ -179,3 +179,31 @@ def test_lines_of_many_or_large_images(gpu, box, N, n):
     o.insert(sl, rots, w, "nearest_neighbor", "c1")
     assert oracle.rel_l2(nm, o.norm) < 2e-6
     assert oracle.rel_l2(d, o.data) < RTOL
+
+
+@pytest.mark.parametrize("box,N,n", [(101, 152, 24), (90, 136, 55), (113, 170, 40), (152, 228, 31)])
+def test_radices_17_and_19_from_24_particles(gpu, box, N, n):
+    """The one-launch preparation of sizes with a factor 17 or 19, which takes
+    over at 24 particles, with and without a phase flip in one call (and without
+    astigmatism, so that no sign hangs on the last place of an angle)."""
+    from eman2_b200 import Reconstructors
+    from eman2_b200.particles import particle_meta
+    from eman2_b200.synth import quaternion_blocks, random_quaternions
+    rng = np.random.default_rng(N + n)
+    img = (rng.normal(size=(n, box, box)) + 3.0).astype(np.float32)
+    rots = quaternion_blocks(random_quaternions(n, rng))
+    shifts = rng.uniform(-3, 3, (n, 2)).astype(np.float32)
+    w = rng.uniform(0.5, 1.0, n).astype(np.float32)
+    df = rng.uniform(0.8, 2.5, n).astype(np.float32)
+    df[::5] = 0.0
+    ctf = {"voltage": 300.0, "cs": 2.7}
+    r = Reconstructors.get("fourier", {"size": [N] * 3, "sym": "c1", "mode": "gauss_2"})
+    r.setup()
+    r.insert_particles(img, particle_meta(rots, shifts, w, ctf=ctf, defocus=df))
+    d, nm = r.get_accumulators()
+    sl = np.stack([oracle.particle_to_slice(img[i], N, shifts[i], dict(ctf, defocus=float(df[i])))
+                   for i in range(n)])
+    o = oracle.OracleVolume(N, "fp32acc64")
+    o.insert(sl, rots, w, "gauss_2", "c1")
+    assert oracle.rel_l2(nm, o.norm) < 2e-6
+    assert oracle.rel_l2(d, o.data) < RTOL
