@@ -41,12 +41,16 @@ Shared *of_current_device() {
   return &g_shared[dev];
 }
 
-// Room for `bytes`, zeroed on st when new; false: none, and nothing held.
+// Room for `bytes`, more than there was, zeroed on st; false: not to be had (a
+// smaller volume stays where it is clear beforehand).
 bool grow(Shared &s, size_t bytes, cudaStream_t st) {
-  s.drop();
   size_t free = 0, total = 0;
-  if (cudaMemGetInfo(&free, &total) == cudaSuccess && bytes <= free / 4 * 3 &&
-      cudaMalloc(&s.p, bytes) == cudaSuccess) {
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess || bytes > (free + s.cap) / 4 * 3) {
+    cudaGetLastError();
+    return false;
+  }
+  s.drop();
+  if (cudaMalloc(&s.p, bytes) == cudaSuccess) {
     s.cap = bytes;
     if (cudaMemsetAsync(s.p, 0, bytes, st) == cudaSuccess) return true;
   } else {

@@ -112,6 +112,24 @@ def test_without_room_straight_into_the_sums(gpu):
     r.close()
 
 
+def test_a_call_too_large_leaves_a_smaller_volume(gpu):
+    """Calls that find no room do not make the others allocate theirs anew."""
+    small, large = _inputs(192, 600), _inputs(256, 800)
+    recons = [_recon(192), _recon(256)]
+    with _left(20 * MB), pytest.raises(Exception):
+        _recon(512)
+    for r, (d_sl, _, rots, w) in zip(recons, (small, large)):
+        r.insert_slices(d_sl[:250], rots[:250], w[:250])    # scratch in place
+    recons[0].insert_slices(small[0], small[2], small[3])
+    with _left(100 * MB):                                   # 57 MB are lent already, 135 would be
+        before = _free()
+        for r, (d_sl, _, rots, w) in zip(recons[::-1], (large, small)):
+            r.insert_slices(d_sl, rots, w)
+        assert abs(before - _free()) < 16 * MB
+    for r in recons:
+        r.close()
+
+
 def test_threads_on_their_own_streams(gpu):
     sizes = (96, 160, 128, 192)
     jobs = [(N, *_inputs(N, 530, 2)) for N in sizes]
